@@ -210,6 +210,9 @@ struct FrameDev {
     uint32_t cullCtasPerSm = 0;        // cap on the persistent tile cull's resident CTAs per SM (0: occupancy)
     uint32_t cullPersistent = 1;       // 0: each tile-cull warp culls one tile, and the grid covers all tiles
     uint32_t streamTiles = 0;          // pipelined launches: the first streamTiles tiles of the queue stream
+    uint32_t* bigCountOut = nullptr;   // [kRateClasses][2] large and huge tiles at the front of each class's order (written with it)
+    const uint32_t* bigCount = nullptr; // the launch's class's entries of it, and the class's tiles before the launch's first
+    uint32_t bigSkip = 0;
 };
 
 
@@ -220,18 +223,19 @@ int setLastError(int code, const char* msg);
 // 12 + log2(msaa) for pinhole views with the rotated-grid pattern
 enum : uint32_t { kRateClasses = 18 };
 // counters: [0] chunk allocator, [1] status, then per tile-cull launch k (2 per rate class)
-// three words at kQueueBase + 3k: work-queue head, retry count, retry-queue head
+// four words at kQueueBase + 4k: work-queue head, retry count, retry-queue head, large tiles' queue head
 // then one word counting the list entries that survive the intersect's per-tile tests, one counting
 // the (warp, surviving entry) pairs whose subsample tests ran (the rest were skipped by the per-warp
 // depth bound), then per launch part k (2 per rate class) the ready-slot tail of its cull -> shade
 // pipeline
 enum : uint32_t {
     kQueueBase = 2,
-    kQueueWords = 3,
+    kQueueWords = 4,
     kSurvivorWord = kQueueBase + kQueueWords * 2 * kRateClasses,
     kTestedWord = kSurvivorWord + 1,
     kPipeBase = kTestedWord + 1,
-    kCounterWords = kPipeBase + 2 * kRateClasses
+    kBigBase = kPipeBase + 2 * kRateClasses, // per rate class: its large and its huge tiles (tileOrderKernel)
+    kCounterWords = kBigBase + 2 * kRateClasses
 };
 
 // kernel launchers (defined in the .cu files); each returns cudaGetLastError()
@@ -263,7 +267,7 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
                                uint32_t* queues, uint32_t warps, uint32_t stackLimit, uint32_t* ready,
                                uint32_t* readyTail, cudaStream_t st);
 cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
-                                    uint32_t* queues, cudaStream_t st);
+                                    uint32_t* queues, uint32_t stackLimit, cudaStream_t st);
 cudaError_t launchCullShadePipeline(const FrameDev& fr, uint32_t msaa, uint32_t pattern, bool fpStrict, uint32_t first,
                                     uint32_t count, uint32_t* queues, uint32_t* pipe, uint32_t warps,
                                     uint32_t stackLimit, cudaStream_t st);

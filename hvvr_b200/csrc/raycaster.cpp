@@ -661,7 +661,7 @@ int ensureSideStreams(hvvr_batch* b) {
     for (uint32_t r = 0; r < kRateClasses; r++) {
         if (!b->rateTiles[r]) continue;
         // the heavy part's stream only where a heavy part can run
-        const bool heavy = b->cfg.heavy_divisor != 0 && !(r >= 6 && r < 12);
+        const bool heavy = b->cfg.tile_stack_entries != 0 && b->cfg.heavy_divisor != 0 && !(r >= 6 && r < 12);
         if (b->side[2 * r + 1] && (b->side[2 * r] || !heavy)) continue;
         if (leastPriority == 0 && greatestPriority == 0)
             CUDA_TRY(cudaDeviceGetStreamPriorityRange(&leastPriority, &greatestPriority));
@@ -740,6 +740,11 @@ int checkStatus(const hvvr_batch* b) {
 }
 
 uint32_t heavyTiles(const hvvr_batch* b, uint32_t n) {
+    // The breadth-first cull takes the large tiles first and finishes each within tens of microseconds,
+    // so a part of their own only adds launches (57k triangles, 640 x 480: 338 us a frame with the
+    // part, 309 without; 1M triangles stereo: 3.38 and 3.30 ms): the heavy part is the sequential
+    // cull's (tile_stack_entries), whose longest tiles take milliseconds.
+    if (!b->cfg.tile_stack_entries) return 0;
     if (!b->costValid || !b->cfg.heavy_divisor || n < kSplitMinTiles) return 0;
     return std::max<uint32_t>(1u, n / b->cfg.heavy_divisor);
 }
@@ -773,7 +778,9 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
         CUDA_TRY(cudaEventRecord(b->orderForkEv, st));
         CUDA_TRY(cudaStreamWaitEvent(os, b->orderForkEv, 0));
     }
-    CUDA_TRY(launchTileOrder(fr, os));
+    FrameDev fo = fr;
+    fo.bigCountOut = fr.counters + kBigBase;
+    CUDA_TRY(launchTileOrder(fo, os));
     if (os != st) CUDA_TRY(cudaEventRecord(b->orderDoneEv, os));
     CUDA_TRY(launchBlockCull(fr, st));
     if (stages) CUDA_TRY(recordStage(b->ev[1], st, capturing));
@@ -782,6 +789,13 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     bool first = true;
     for (auto& u : b->kevUsed) u = false;
     for (auto& u : b->kevPipelined) u = false;
+    // the frame as the tile cull of class r sees it, `skip` tiles into the class
+    auto part1 = [](const FrameDev& f, uint32_t r, uint32_t skip) {
+        FrameDev p = f;
+        p.bigCount = f.counters + kBigBase + 2 * r;
+        p.bigSkip = skip;
+        return p;
+    };
     // Pinhole classes: per part, tile cull then intersect on the part's stream, or (config.pipeline)
     // one cull -> shade pipeline per part. Thin-lens classes (one part each) need the occupied-tile
     // ranks of the whole view, so all their culls finish before one rank launch, and their
@@ -799,9 +813,12 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             cudaStream_t ps = b->side[k];
             CUDA_TRY(cudaStreamWaitEvent(ps, b->forkEv, 0));
             if (stages) CUDA_TRY(recordStage(b->kev[k][0], ps, capturing));
-            if (!lens && b->cfg.pipeline) {
+            // From 16 subsamples the shade is several times as long as the breadth-first cull, and its
+            // CTAs are better used from the cull's end, longest tile first, than waiting for tiles.
+            const bool piped = b->cfg.pipeline && (msaa < 16 || b->cfg.tile_stack_entries);
+            if (!lens && piped) {
                 // the class's first part holds its longest tiles: those stream their lists
-                FrameDev fp = fr;
+                FrameDev fp = part1(fr, r, p0 - rs);
                 fp.streamTiles = part == (heavy ? 0u : 1u) ? b->cfg.stream_tiles : 0u;
                 CUDA_TRY(launchCullShadePipeline(fp, msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                                  fr.counters + kPipeBase + k, b->cfg.tile_cull_warps,
@@ -819,7 +836,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
                 CUDA_TRY(cudaStreamWaitEvent(st, b->doneEv[k], 0));
                 continue;
             }
-            CUDA_TRY(launchTileCull(fr, fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
+            CUDA_TRY(launchTileCull(part1(fr, r, p0 - rs), fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                     b->cfg.tile_cull_warps, b->cfg.tile_stack_entries, ps));
             if (stages) CUDA_TRY(recordStage(b->kev[k][1], ps, capturing));
             if (stages && part == 1 && first) CUDA_TRY(recordStage(b->ev[2], ps, capturing));

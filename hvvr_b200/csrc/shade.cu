@@ -1300,7 +1300,7 @@ cudaError_t launchPipelineRate(const FrameDev& fr, uint32_t first, uint32_t coun
     if ((e = cudaLaunchKernelEx(&cfg, intersectShadeKernel<N, FMA, kFromReady, ROW>, fr, ready)) != cudaSuccess) return e;
     // tiles whose stack outgrew the main pass: culled again, then shaded by a small grid that walks
     // the retry list (its length is only known on the device)
-    if ((e = launchTileCullRetryPass(fr, fr.order, first, count, queues, st)) != cudaSuccess) return e;
+    if ((e = launchTileCullRetryPass(fr, fr.order, first, count, queues, stackLimit, st)) != cudaSuccess) return e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

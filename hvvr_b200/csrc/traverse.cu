@@ -1,15 +1,18 @@
 // traverse.cu - tile-frustum BVH traversal on the GPU.
 //
-// Two kernels restate the reference's two-level CPU traversal (cullThread,
-// libraries/hvvr/raycaster/traversal.cpp:99-190) one warp per frustum:
+// The reference's two-level CPU traversal (cullThread, libraries/hvvr/raycaster/traversal.cpp:99-190):
 //   blockCullKernel: traverseBlocks + BlockFrame::sort per 8192-sample block frustum
-//                    (libraries/hvvr/raycaster/traverse_avx.h:293-410);
-//   tileCullKernel:  traverseTiles per 128-sample tile frustum, starting from its block's
-//                    sorted stack (traverse_avx.h:412-527), emitting the tile's triangle list.
-// Both rebuild the world-space frustum of Frustum::Frustum (traverse_avx.cpp:22-211) from the
+//                    (libraries/hvvr/raycaster/traverse_avx.h:293-410), one warp each;
+//   tileTreeKernel, tileTreeHugeKernel: traverseTiles per 128-sample tile frustum, starting from its
+//                    block's sorted stack (traverse_avx.h:412-527), emitting the tile's triangle list:
+//                    the nodes visited breadth first, the list's order recovered afterwards;
+//   tileCullKernel:  the same as the reference runs it, node by node with a sorted stack, one warp per
+//                    tile: what the breadth-first cull leaves (above 8,192 visits, bounds that do not
+//                    nest) and callers that set the stack's size (tile_stack_entries).
+// All rebuild the world-space frustum of Frustum::Frustum (traverse_avx.cpp:22-211) from the
 // camera-space corner rays and the camera matrix (frustumTransform, traversal.h:38-47).
 //
-// Lane layout of one node visit: lane l loads word l of the 128-byte node (one coalesced
+// Lane layout of one sequential node visit: lane l loads word l of the 128-byte node (one coalesced
 // row); child c = l & 3 receives its six bounds by shuffle. Lanes 0-15 run the plane test
 // of plane l>>2, lanes 16-27 the axis-projection test of axis (l-16)>>2, and every lane runs
 // one or two of the 48 edge-axis tests (edge l>>2 and, for l < 16, edge 8+(l>>2)). Ballots
@@ -276,6 +279,15 @@ __device__ __forceinline__ bool edgeReject(const ChildBox& b, float ex, float ey
     const float maxBox = fmaf(ex, pX, fmaf(ey, pY, ez * pZ));
     const float minBox = fmaf(ex, nX, fmaf(ey, nY, ez * nZ));
     return (maxBox < mn) || (mx < minBox);
+}
+
+// edgeReject for an edge axis with a zero component, without that component's (zero) product: e.x and
+// e.y are the other two components, e.z and e.w the frustum's range along the axis
+__device__ __forceinline__ bool edgeReject2(float aM, float aN, float bM, float bN, float4 e) {
+    const bool pa = e.x > 0.0f, pb = e.y > 0.0f;
+    const float maxBox = fmaf(e.x, pa ? aM : -aN, e.y * (pb ? bM : -bN));
+    const float minBox = fmaf(e.x, pa ? -aN : aM, e.y * (pb ? -bN : bM));
+    return (maxBox < e.z) | (e.w < minBox);
 }
 
 // Frustum::testBVHNodeChildrenRefine (traverse_avx.h:166-217): mask of rejected children
@@ -603,6 +615,14 @@ struct TileCullArgs {
     uint32_t* readyTail;   // pipelined: finished tiles so far, zero at launch
     uint32_t persistent;   // 0: every warp culls one tile (the grid has a warp per tile), then exits
     uint32_t streamTiles;  // with ready: queue positions below this stream their lists (else 0)
+    const uint32_t* counts; // breadth-first cull: the large, and of those the huge, tiles at the front of the rate
+                           // class's order (nullptr: none)
+    uint32_t skip;         // tiles of the class before `first`
+    uint32_t* bigQueue;    // work-queue head of the large tiles, zero at launch
+
+    __device__ uint32_t front(uint32_t n) const { return n > skip ? min(n - skip, count) : 0u; }
+    __device__ uint32_t big() const { return counts ? front(__ldcg(counts)) : 0u; }
+    __device__ uint32_t huge() const { return counts ? front(__ldcg(counts + 1)) : 0u; }
 };
 
 // traverseTiles for one tile of view V (tile = view-local index); returns the node visits.
@@ -891,56 +911,760 @@ __global__ void __launch_bounds__(W * 32, W == 1 ? 20 : 1) tileCullKernel(TileCu
     }
 }
 
-// The tiles whose sorted stack outgrew kTileStack, culled again from the start with the
-// reference's TileFrame capacity (4096 entries, 48 KiB of shared memory per warp).
+// ---------------------------------------------------------------- breadth-first tile cull
+// traverseTiles without its serial chain of node visits. The traversal has no early out: it visits
+// every node whose ancestors pass the tile's tests, and its sorted stack only decides the order in
+// which the passing leaves' triangles enter the list. So the nodes are visited breadth first, eight
+// per warp step (lane = node * 4 + child), and the order is recovered afterwards:
+//
+//   The stack pops the smallest key, newest first among equal keys, and a node with a single
+//   passing child goes to it at once (an edge of key -infinity). For two visited nodes a and b with
+//   lowest common ancestor L, a comes first when the largest key on the path from L to a is smaller
+//   than the one on the path to b (the element that holds b's maximum cannot be popped while
+//   anything on a's path is pending); with equal maxima, the first elements that hold them were
+//   pushed when their parents were popped, and the one pushed later is popped first - so the order
+//   of the parents, reversed (or the later slot, for siblings).
+//   Child boxes nest, so keys do not fall along a path, and the nodes form connected components: a
+//   component's head is a child of a node with several passing children, with a key above its
+//   parent's component's; a child with an equal key, and a single child, belong to the parent's
+//   component. A component is popped without interruption, in depth-first order, later slots first.
+//   The block's stack entries are the roots; their keys may be measured along another axis than the
+//   tile's, so a root's key takes part only in comparisons between different roots.
+//
+// Components with passing leaves are sorted by (largest key on the path, then compBefore), and a
+// node's place is its component's start plus its depth-first offset. A tile that does not fit the
+// store, or whose keys fall along a path (bounds that do not nest, NaN), is left to the sequential
+// kernels, which give the same list for every input.
+//
+// What bounds it: issue and the barriers between generations (54% of the issue slots, ncu), with about
+// 60 instructions per visit; eight warps per large tile and four CTAs (64 registers) per SM keep both
+// short chains and enough warps. The sequential traversal is a chain of about 2,000 cycles per visit.
+// The cull launch alone, before and after, one B200: 57k triangles 640 x 480, 229 and 81 us; 1M
+// triangles 1280 x 720, 3,364 and 371 us; 1M triangles stereo 2 x 1080 x 1200, 2,511 and 978 us. With
+// two CTAs of 128 registers per SM the last took 1,255 us.
+constexpr uint32_t kTreeWarps = 8;
+constexpr uint32_t kWarpNodes = 256;                       // visited nodes of a tile culled by one warp,
+constexpr uint32_t kCtaNodes = kTreeWarps * kWarpNodes;    // of one culled by a CTA of 8 warps,
+constexpr uint32_t kHugeWarps = 16, kHugeNodes = 8192;     // and by a CTA of 16 warps that has an SM for itself
+constexpr uint32_t kMaxGens = 64;
 constexpr uint32_t kRetryStack = 4096;
-__global__ void __launch_bounds__(32) tileCullRetryKernel(TileCullArgs a) {
-    extern __shared__ __align__(16) unsigned char retrySmem[];
-    TileSmemT<kRetryStack>& s = *reinterpret_cast<TileSmemT<kRetryStack>*>(retrySmem);
-    const uint32_t lane = laneId();
+constexpr uint32_t kMaxLeafRange = 65535;                  // longer leaf ranges are left to the sequential kernels
+
+// A component is named by its head's store index.
+template <uint32_t N>
+struct TreeStore {
+    static constexpr uint32_t kNodes = N, kSorted = N / 2;
+    unsigned long long sortKey[kSorted]; // largest key on the path << 32 | component; later list staging
+    uint32_t node[N];
+    uint32_t key[N];        // order key of a component's head, 0 for a root's
+    uint32_t meta[N];       // kMeta... below
+    uint16_t first[N];      // first child; later the nodes in traversal order
+    uint16_t comp[N];
+    uint16_t size[N];       // nodes of the component at and below the node, then the depth-first offset
+    uint16_t compSize[N];   // of heads; then the component's first position
+};
+// meta: a head's parent (bits 0-12), root index (13-18), whether its component has passing leaves
+// (19); a node's passing leaf slots (20-23) and internal children (24-26); a root that stands for
+// leaf slots only (27)
+constexpr uint32_t kMetaParent = 0x1fffu, kMetaRoot = 13, kMetaLeafy = 1u << 19, kMetaSlots = 20, kMetaChildren = 24,
+                   kMetaMasked = 1u << 27;
+static_assert(kHugeNodes <= kMetaParent + 1, "parent index bits");
+static_assert(sizeof(TreeStore<kWarpNodes>::sortKey) >= sizeof(SmemFrustum), "the frustum is built in the sort's memory");
+
+struct TreeHead {
+    float4 lo[4], hi[4];     // frustum planes: tpLo, w | tpHi
+    float4 edge[12];         // edge axes, the two components that the cross product with an axis leaves; min, max
+    uint32_t rootKey[kBlockStack];
+    uint16_t gen[kMaxGens + 2]; // generation g is nodes [gen[g], gen[g + 1])
+    uint32_t pushed[3];      // nodes pushed in a generation (in turn), kPushedBad added where the tile cannot be culled here
+    uint32_t total, first, sorted;
+    uint32_t warpSum[kHugeWarps];
+};
+constexpr uint32_t kPushedBad = 1u << 20;
+
+struct TreeSmem {
+    TreeHead head[kTreeWarps];
+    union {
+        TreeStore<kWarpNodes> warp[kTreeWarps];
+        TreeStore<kCtaNodes> cta;
+    };
+    uint32_t item, spill;
+};
+struct HugeSmem {
+    TreeHead head;
+    union {
+        TreeStore<kHugeNodes> cta;
+        TileSmemT<kRetryStack> seq;
+    };
+    uint32_t item;
+};
+
+// a float's order under the denormals-are-zero comparison, as an unsigned integer above 0 (NaN excepted)
+__device__ __forceinline__ uint32_t orderKey(float v) {
+    uint32_t u = __float_as_uint(v);
+    if ((u & 0x7f800000u) == 0) u = 0;
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// whether component a is popped before component b (see above); called where the sort keys are equal
+template <class S>
+__device__ __noinline__ bool compBefore(const S& s, const uint32_t* rootKey, uint32_t a, uint32_t b) {
+    bool flip = false;
     for (;;) {
-        uint32_t w = 0;
-        if (lane == 0) w = atomicAdd(a.retryQueue, 1u);
-        w = __shfl_sync(kFull, w, 0);
-        if (w >= *reinterpret_cast<volatile uint32_t*>(a.retryCount)) return;
-        const uint32_t gt = a.retry[a.first + w];
-        const ViewDev& V = viewOfBlock(a.views, a.blockView, a.viewCount, gt / kTilesPerBlock);
-        const uint32_t tile = gt - V.tileStart;
-        __syncwarp();
-        bool overflow;
-        const uint32_t visits = cullTile(a, V, tile, s, overflow);
-        if (lane == 0) {
-            V.tileCost[tile] = visits;
-            if (overflow) atomicOr(&a.counters[1], kStatusStackOverflow);
+        const uint32_t ma = s.meta[a], mb = s.meta[b], ka = s.key[a], kb = s.key[b];
+        const uint32_t ra = (ma >> kMetaRoot) & 63u, rb = (mb >> kMetaRoot) & 63u;
+        const bool sameRoot = ra == rb;
+        const uint32_t ea = sameRoot ? ka : max(rootKey[ra], ka), eb = sameRoot ? kb : max(rootKey[rb], kb);
+        if (ea != eb) return (ea < eb) != flip;
+        if (!sameRoot) {
+            // a root that holds its path's maximum was there from the start: below anything pushed
+            // since, and roots in stack order
+            const bool la = rootKey[ra] >= ka, lb = rootKey[rb] >= kb;
+            if (la || lb) return (la && lb ? ra > rb : lb) != flip;
         }
-        __syncwarp();
+        const uint32_t pa = ma & kMetaParent, pb = mb & kMetaParent;
+        const uint32_t ca = s.comp[pa], cb = s.comp[pb];
+        if (ca == cb) return (pa != pb ? s.size[pa] > s.size[pb] : a > b) != flip;
+        a = ca;
+        b = cb;
+        flip = !flip;
     }
 }
 
-// Orders the global tiles by (rate class ascending, cost descending), cost in log2 buckets
-// of last frame's visit counts. One block; positions within a bucket are in arrival order.
-constexpr uint32_t kOrderBuckets = kRateClasses * 33;
+__device__ __forceinline__ uint32_t warpInclusive(uint32_t v) {
+    const uint32_t lane = laneId();
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, v, o);
+        if (lane >= o) v += y;
+    }
+    return v;
+}
+
+// ascending compare-exchange of v with lane ^ mask's
+__device__ __forceinline__ unsigned long long laneExchange(unsigned long long v, uint32_t mask) {
+    const unsigned long long o = __shfl_xor_sync(kFull, v, mask);
+    const bool low = laneId() < (laneId() ^ mask);
+    return (v < o) == low ? v : o;
+}
+
+// Ascending sort of n 64-bit values in shared memory by the group's warps: blocks of 32 in
+// registers, then a bitonic network whose comparisons are all ascending (positions past the end
+// need no padding), its strides below 32 in registers again.
+template <int W, class Sync>
+__device__ void groupSort(unsigned long long* v, uint32_t n, uint32_t wid, Sync sync) {
+    constexpr uint32_t G = 32 * W;
+    const uint32_t lane = laneId(), tid = wid * 32 + lane;
+    for (uint32_t b = wid * 32; b < n; b += G) {
+        unsigned long long x = b + lane < n ? v[b + lane] : ~0ull;
+#pragma unroll
+        for (uint32_t k = 2; k <= 32; k <<= 1) {
+            x = laneExchange(x, k - 1);
+#pragma unroll
+            for (uint32_t d = k >> 2; d > 0; d >>= 1) x = laneExchange(x, d);
+        }
+        if (b + lane < n) v[b + lane] = x;
+    }
+    sync();
+    auto order2 = [&](uint32_t i, uint32_t j) {
+        if (j >= n) return;
+        const unsigned long long x = v[i], y = v[j];
+        if (y < x) {
+            v[i] = y;
+            v[j] = x;
+        }
+    };
+    for (uint32_t half = 32; half < n; half <<= 1) {
+        for (uint32_t t = tid; (t & ~(half - 1)) * 2 < n; t += G) {
+            const uint32_t low = t & (half - 1), block = (t - low) * 2;
+            order2(block + low, block + 2 * half - 1 - low);
+        }
+        sync();
+        for (uint32_t d = half >> 1; d >= 32; d >>= 1) {
+            for (uint32_t t = tid; (t & ~(d - 1)) * 2 < n; t += G) {
+                const uint32_t low = t & (d - 1), block = (t - low) * 2;
+                order2(block + low, block + d + low);
+            }
+            sync();
+        }
+        for (uint32_t b = wid * 32; b < n; b += G) {
+            unsigned long long x = b + lane < n ? v[b + lane] : ~0ull;
+#pragma unroll
+            for (uint32_t d = 16; d > 0; d >>= 1) x = laneExchange(x, d);
+            if (b + lane < n) v[b + lane] = x;
+        }
+        sync();
+    }
+}
+
+// one tile by W warps (W = 1: the calling warp alone; else the whole CTA); returns the node visits.
+// overflow: the list was not made (see above).
+template <int W, uint32_t N>
+__device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t tile, TreeHead& h, TreeStore<N>& s,
+                             bool& overflow) {
+    constexpr uint32_t G = 32 * W;
+    using S = TreeStore<N>;
+    const uint32_t lane = laneId(), wid = W == 1 ? 0u : threadIdx.x >> 5, tid = W == 1 ? lane : threadIdx.x;
+    const uint32_t q4 = lane & 28u, c = lane & 3u, below = (1u << lane) - 1u;
+    auto sync = [] {
+        if constexpr (W == 1) __syncwarp();
+        else __syncthreads();
+    };
+    overflow = false;
+    const uint32_t blk = tile / kTilesPerBlock;
+    const uint32_t roots = V.blockSizes[blk];
+    SmemFrustum& f = *reinterpret_cast<SmemFrustum*>(s.sortKey); // until the sort
+    bool bad = false;
+    for (uint32_t i = tid; i < roots; i += G) {
+        const StackEntry e = V.blockStacks[size_t(blk) * kBlockStack + i];
+        s.node[i] = e.node;
+        s.comp[i] = uint16_t(i);
+        s.meta[i] = i | (i << kMetaRoot) | (e.mask ? kMetaMasked : 0u);
+        s.key[i] = 0;
+        h.rootKey[i] = orderKey(e.tMin);
+        if (isnan(e.tMin)) bad = true;
+    }
+    if (wid == 0) {
+        buildFrustum(V.tileRays[tile], V.M, f);
+        if (lane < 4) {
+            h.lo[lane] = make_float4(f.tpLo[lane][0], f.tpLo[lane][1], f.tpLo[lane][2], f.w[lane]);
+            h.hi[lane] = make_float4(f.tpHi[lane][0], f.tpHi[lane][1], f.tpHi[lane][2], 0.0f);
+        } else if (lane < 16) {
+            const uint32_t e = lane - 4, k = e % 3;
+            h.edge[e] = make_float4(f.edge[e][k == 0 ? 1 : 0], f.edge[e][k == 2 ? 1 : 2], f.minF[e], f.maxF[e]);
+            if (!(f.edge[e][k] == 0.0f)) bad = true; // (a direction that is not finite)
+        } else if (lane < 19) {
+            h.pushed[lane - 16] = 0;
+        } else if (lane == 19) {
+            h.total = h.sorted = 0;
+            h.gen[0] = 0;
+        }
+    }
+    const bool culled = V.hasCull && tileCulled(V.tileRays[tile], V.M, V.cull);
+    sync();
+    if (culled || roots == 0 || f.degenerate) {
+        if (tid == 0) V.tileLists[tile] = TileList{kNoChunk, 0};
+        sync();
+        return 0;
+    }
+    // the stack is sorted from the farthest up (a caller's own block stacks may not be)
+    for (uint32_t i = tid; i + 1 < roots; i += G)
+        if (h.rootKey[i] < h.rootKey[i + 1]) bad = true;
+    const int distIdx = f.distIdx;
+    const float p0 = f.proj[0][c], p1 = f.proj[0][4 + c], p2 = f.proj[1][c], p3 = f.proj[1][4 + c],
+                p4 = f.proj[2][c], p5 = f.proj[2][4 + c];
+    const float* rows = reinterpret_cast<const float*>(V.nodes);
+
+    uint32_t lo = 0, hi = roots, gens = 0, total = 0;
+    for (;;) {
+        uint32_t next = hi; // (W = 1) end of the next generation so far
+        for (uint32_t base = lo + wid * 8; base < hi; base += 8 * W) {
+            const uint32_t i = base + (lane >> 2);
+            const bool act = i < hi;
+            const uint32_t n = act ? s.node[i] : 0u;
+            const uint32_t meta = act ? s.meta[i] : 0u;
+            const float* row = rows + size_t(n) * 32;
+            ChildBox b{};
+            uint32_t leafMask = 0, t0 = 0, t1 = 0;
+            if (act) {
+                b = ChildBox{row[c], row[4 + c], row[8 + c], row[12 + c], row[16 + c], row[20 + c]};
+                leafMask = __float_as_uint(row[24]);
+                t0 = __float_as_uint(row[25 + c]);
+                t1 = __float_as_uint(row[26 + c]);
+            }
+            // testBVHNodeChildren
+            bool pass = act & (b.xM >= p0) & (b.xN >= p1) & (b.yM >= p2) & (b.yN >= p3) & (b.zM >= p4) & (b.zN >= p5);
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                const float4 l = h.lo[p], u = h.hi[p];
+                const float dl = fmaf(l.x, b.xM, fmaf(l.y, b.yM, l.z * b.zM));
+                const float du = fmaf(u.x, b.xN, fmaf(u.y, b.yN, u.z * b.zN));
+                pass = pass & ((dl + du) <= l.w);
+            }
+            // testBVHNodeChildrenRefine, for every child of a node with a passing leaf
+            const bool leafy = ((__ballot_sync(kFull, pass) >> q4) & 15u & leafMask) != 0;
+            const bool refine = pass & leafy;
+            if (__any_sync(kFull, refine)) {
+                bool reject = false;
+#pragma unroll
+                for (int e = 0; e < 12; e += 3) {
+                    const float4 ex = h.edge[e], ey = h.edge[e + 1], ez = h.edge[e + 2];
+                    reject = reject | edgeReject2(b.yM, b.yN, b.zM, b.zN, ex) | edgeReject2(b.xM, b.xN, b.zM, b.zN, ey) |
+                             edgeReject2(b.xM, b.xN, b.yM, b.yN, ez);
+                }
+                pass = pass & !(refine & reject);
+                // a zero component's product is zero (so edgeReject2 can leave it out) only for finite bounds
+                if (refine && !(fabsf(((b.xM + b.xN) + (b.yM + b.yN)) + (b.zM + b.zN)) <= FLT_MAX)) bad = true;
+            }
+            const bool leaf = (leafMask >> c) & 1u;
+            uint32_t len = 0;
+            if (pass & leaf) {
+                if (t1 <= t0) {
+                    atomicOr(&a.counters[1], kStatusBadLeaf);
+                } else {
+                    len = t1 - t0;
+                    if (len > kMaxLeafRange) bad = true, len = 1;
+                }
+            }
+            const uint32_t leafBits = (__ballot_sync(kFull, len != 0) >> q4) & 15u;
+            total += len;
+            // the internal children that pass are the next generation's nodes
+            const bool push = pass & !leaf & !(meta & kMetaMasked);
+            const uint32_t pb = __ballot_sync(kFull, push);
+            const uint32_t m = __popc((pb >> q4) & 15u);
+            uint32_t at = next;
+            if constexpr (W == 1) {
+                next += __popc(pb);
+            } else if (pb) {
+                if (lane == 0) at = hi + atomicAdd(&h.pushed[gens % 3u], uint32_t(__popc(pb)));
+                at = __shfl_sync(kFull, at, 0);
+            }
+            const uint32_t pos = at + __popc(pb & below);
+            const uint32_t comp = act ? s.comp[i] : 0u;
+            if (push & (pos < N)) {
+                uint32_t cid = comp;
+                if (m > 1) {
+                    const float v = distIdx < 2 ? (distIdx == 0 ? b.xM : b.xN)
+                                                : (distIdx < 4 ? (distIdx == 2 ? b.yM : b.yN) : (distIdx == 4 ? b.zM : b.zN));
+                    const uint32_t key = orderKey(-v), parentKey = s.key[comp];
+                    if (key < parentKey || isnan(v)) bad = true;
+                    if (key != parentKey) {
+                        cid = pos;
+                        s.key[pos] = key;
+                    }
+                }
+                s.node[pos] = n + t1;
+                s.comp[pos] = uint16_t(cid);
+                s.meta[pos] = i | (s.meta[comp] & (63u << kMetaRoot));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(rows + size_t(n + t1) * 32));
+            }
+            __syncwarp();
+            if (act & (c == 0)) {
+                s.first[i] = uint16_t(at + __popc(pb & below));
+                atomicOr(&s.meta[i], (leafBits << kMetaSlots) | (m << kMetaChildren));
+                if (leafBits) atomicOr(&s.meta[comp], kMetaLeafy);
+            }
+        }
+        if constexpr (W == 1) {
+            if (__any_sync(kFull, bad)) next = N + 1;
+            __syncwarp();
+        } else {
+            if (bad) atomicAdd(&h.pushed[gens % 3u], kPushedBad);
+            __syncthreads();
+            next = hi + h.pushed[gens % 3u];
+            if (tid == 0) h.pushed[(gens + 2u) % 3u] = 0; // (read before the last barrier, used after the next)
+        }
+        ++gens;
+        if (tid == 0) h.gen[gens] = uint16_t(hi);
+        if (next > N || (gens >= kMaxGens && next != hi)) {
+            overflow = true;
+            sync();
+            return min(hi, N);
+        }
+        if (next == hi) break;
+        lo = hi;
+        hi = next;
+    }
+    const uint32_t visits = hi;
+    total = __reduce_add_sync(kFull, total);
+    if constexpr (W > 1) {
+        if (lane == 0 && total) atomicAdd(&h.total, total);
+        __syncthreads();
+        total = h.total;
+    }
+    if (total == 0) {
+        if (tid == 0) V.tileLists[tile] = TileList{kNoChunk, 0};
+        sync();
+        return visits;
+    }
+    // the list's chunks, consecutive in the pool
+    const uint32_t chunks = (total + kChunk - 1) / kChunk;
+    uint32_t chunk0 = 0;
+    if (tid == 0) {
+        chunk0 = atomicAdd(&a.counters[0], chunks);
+        if (W > 1) h.first = chunk0;
+    }
+    __syncwarp();
+    // depth-first offsets inside the components: subtree sizes upwards, offsets downwards
+    for (uint32_t g = gens; g-- > 0;) {
+        for (uint32_t i = h.gen[g] + tid; i < h.gen[g + 1]; i += G) {
+            const uint32_t m = (s.meta[i] >> kMetaChildren) & 7u, fc = s.first[i], own = s.comp[i];
+            uint32_t z = 1;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                if (k < m && s.comp[fc + k] == own) z += s.size[fc + k];
+            s.size[i] = uint16_t(z);
+            if (g == 0) s.compSize[i] = uint16_t(z);
+        }
+        sync();
+    }
+    for (uint32_t i = tid; i < roots; i += G) s.size[i] = 0;
+    sync();
+    for (uint32_t g = 0; g + 1 < gens; g++) {
+        for (uint32_t i = h.gen[g] + tid; i < h.gen[g + 1]; i += G) {
+            const uint32_t m = (s.meta[i] >> kMetaChildren) & 7u, fc = s.first[i], own = s.comp[i];
+            uint32_t off = s.size[i] + 1u, z[4], cid[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                z[k] = k < m ? s.size[fc + k] : 0u;
+                cid[k] = k < m ? s.comp[fc + k] : 0u;
+            }
+#pragma unroll
+            for (int k = 3; k >= 0; k--) {
+                if (uint32_t(k) >= m) continue;
+                if (cid[k] == own) {
+                    s.size[fc + k] = uint16_t(off);
+                    off += z[k];
+                } else {
+                    s.compSize[cid[k]] = uint16_t(z[k]);
+                    s.size[fc + k] = 0;
+                }
+            }
+        }
+        sync();
+    }
+    // the components with passing leaves, by largest key on the path
+    uint32_t sorted = 0;
+    for (uint32_t b = wid * 32; b < visits; b += G) {
+        const uint32_t i = b + lane;
+        const uint32_t meta = i < visits && s.comp[i] == i ? s.meta[i] : 0u;
+        const uint32_t on = __ballot_sync(kFull, meta & kMetaLeafy);
+        uint32_t pos = sorted;
+        if constexpr (W == 1) {
+            sorted += __popc(on);
+        } else if (on) {
+            if (lane == 0) pos = atomicAdd(&h.sorted, uint32_t(__popc(on)));
+            pos = __shfl_sync(kFull, pos, 0);
+        }
+        pos += __popc(on & below);
+        if ((meta & kMetaLeafy) && pos < S::kSorted)
+            s.sortKey[pos] = (uint64_t(max(h.rootKey[(meta >> kMetaRoot) & 63u], s.key[i])) << 32) | i;
+    }
+    sync();
+    if constexpr (W > 1) sorted = h.sorted;
+    if (sorted > S::kSorted) {
+        // (its chunks stay allocated and unused)
+        overflow = true;
+        sync();
+        return visits;
+    }
+    groupSort<W>(s.sortKey, sorted, wid, sync);
+    // runs of equal keys in their exact order
+    uint16_t* ordered = s.first;
+    for (uint32_t e = tid; e < sorted; e += G) {
+        const unsigned long long v = s.sortKey[e];
+        const uint32_t key = uint32_t(v >> 32), id = uint32_t(v);
+        uint32_t pos = e;
+        for (uint32_t j = e; j-- > 0;) {
+            const unsigned long long o = s.sortKey[j];
+            if (uint32_t(o >> 32) != key) break;
+            if (!compBefore(s, h.rootKey, uint32_t(o), id)) pos--;
+        }
+        for (uint32_t j = e + 1; j < sorted; j++) {
+            const unsigned long long o = s.sortKey[j];
+            if (uint32_t(o >> 32) != key) break;
+            if (compBefore(s, h.rootKey, uint32_t(o), id)) pos++;
+        }
+        ordered[pos] = uint16_t(id);
+    }
+    sync();
+    // the components' first positions
+    uint32_t placed = 0;
+    for (uint32_t b = 0; b < sorted; b += G) {
+        const uint32_t j = b + tid;
+        const uint32_t cid = j < sorted ? ordered[j] : 0u;
+        const uint32_t z = j < sorted ? s.compSize[cid] : 0u;
+        const uint32_t inc = warpInclusive(z);
+        uint32_t start = placed;
+        if constexpr (W > 1) {
+            if (lane == 31) h.warpSum[wid] = inc;
+            __syncthreads();
+            uint32_t all = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < uint32_t(W); w++) {
+                if (w < wid) start += h.warpSum[w];
+                all += h.warpSum[w];
+            }
+            placed += all;
+            __syncthreads();
+        } else {
+            placed += __shfl_sync(kFull, inc, 31);
+        }
+        if (j < sorted) s.compSize[cid] = uint16_t(start + inc - z);
+    }
+    sync();
+    uint16_t* at = s.first;
+    for (uint32_t i = tid; i < visits; i += G) {
+        const uint32_t cid = s.comp[i];
+        if (s.meta[cid] & kMetaLeafy) at[s.compSize[cid] + s.size[i]] = uint16_t(i);
+    }
+    if constexpr (W == 1) chunk0 = __shfl_sync(kFull, chunk0, 0);
+    else chunk0 = h.first;
+    sync();
+    if (chunk0 >= a.poolChunks || chunks > a.poolChunks - chunk0) {
+        if (tid == 0) {
+            atomicOr(&a.counters[1], kStatusPoolOverflow);
+            V.tileLists[tile] = TileList{kNoChunk, 0};
+        }
+        sync();
+        return visits;
+    }
+    for (uint32_t k = tid; k < chunks; k += G) a.chunkNext[chunk0 + k] = k + 1 < chunks ? chunk0 + k + 1 : kNoChunk;
+    // the list: groups of 32 nodes in order, a lane per node; a group's entries are gathered in shared
+    // memory (the sort's) and written out together
+    uint32_t* out = a.pool + size_t(chunk0) * kChunk;
+    constexpr uint32_t kStageEntries = 2 * S::kSorted / W;
+    uint32_t* stage = reinterpret_cast<uint32_t*>(s.sortKey) + wid * kStageEntries;
+    uint32_t* groupAt = s.key; // (its last use was the runs' order)
+    const uint32_t groups = (placed + 31) / 32;
+    struct Leaves {
+        uint32_t t[5], bits, count;
+    };
+    auto leavesOf = [&](uint32_t g) {
+        Leaves r;
+        r.bits = r.count = 0;
+        const uint32_t j = g * 32 + lane;
+        const uint32_t i = j < placed ? at[j] : 0u;
+        if (j < placed) r.bits = (s.meta[i] >> kMetaSlots) & 15u;
+        if (r.bits) {
+            const uint4* w = reinterpret_cast<const uint4*>(rows + size_t(s.node[i]) * 32 + 24);
+            const uint4 w0 = __ldg(w), w1 = __ldg(w + 1);
+            r.t[0] = w0.y; r.t[1] = w0.z; r.t[2] = w0.w; r.t[3] = w1.x; r.t[4] = w1.y;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if ((r.bits >> k) & 1u) r.count += r.t[k + 1] - r.t[k];
+        }
+        return r;
+    };
+    if constexpr (W > 1) {
+        for (uint32_t g = wid; g < groups; g += W) {
+            const uint32_t n = __reduce_add_sync(kFull, leavesOf(g).count);
+            if (lane == 0) groupAt[g] = n;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            uint32_t run = 0;
+            for (uint32_t b = 0; b < groups; b += 32) {
+                const uint32_t n = b + lane < groups ? groupAt[b + lane] : 0u;
+                const uint32_t inc = warpInclusive(n);
+                if (b + lane < groups) groupAt[b + lane] = run + inc - n;
+                run += __shfl_sync(kFull, inc, 31);
+            }
+        }
+        __syncthreads();
+    }
+    uint32_t base = 0;
+    for (uint32_t g = wid; g < groups; g += W) {
+        const Leaves r = leavesOf(g);
+        const uint32_t inc = warpInclusive(r.count);
+        const uint32_t n = __shfl_sync(kFull, inc, 31);
+        if constexpr (W > 1) base = groupAt[g];
+        const bool staged = n <= kStageEntries;
+        uint32_t* dst = (staged ? stage : out + base) + (inc - r.count);
+        if (r.bits) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if ((r.bits >> k) & 1u)
+                    for (uint32_t t = r.t[k]; t < r.t[k + 1]; t++) *dst++ = t;
+        }
+        if (staged) {
+            __syncwarp();
+            for (uint32_t e = lane; e < n; e += 32) out[base + e] = stage[e];
+            __syncwarp();
+        }
+        base += n;
+    }
+    if (tid == 0) V.tileLists[tile] = TileList{chunk0, total};
+    return visits;
+}
+
+// Publishes a finished tile to the concurrent shade: every thread's list writes are made visible
+// device-wide before one releases the ready slot.
+template <int W>
+__device__ __forceinline__ void publishTile(const TileCullArgs& a, uint32_t gt, bool retry) {
+    if (!a.ready) return;
+    __threadfence();
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+    if ((W == 1 ? laneId() : threadIdx.x) == 0) {
+        const uint32_t pos = atomicAdd(a.readyTail, 1u);
+        const uint32_t val = gt | (retry ? kReadyRetry : 0u);
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.ready + a.first + pos), "r"(val) : "memory");
+    }
+}
+
+// Persistent CTAs. The tiles that were large in the last frame (a.counts[0] tiles at the front of the
+// class's order, of which the first a.counts[1] are culled by tileTreeHugeKernel) are culled by a whole
+// CTA each, then every warp takes small ones; a small one that outgrows its warp's store is kept in a
+// list of its CTA (linked through the tiles' unwritten TileLists) and culled by the whole CTA once its
+// warps are done. Tiles that outgrow the CTA's store go to the retry list. Non-persistent: a CTA takes
+// one large tile, or one small one per warp.
+__global__ void __launch_bounds__(kTreeWarps * 32, 4) tileTreeKernel(TileCullArgs a) {
+    extern __shared__ __align__(16) unsigned char treeRaw[];
+    TreeSmem& sm = *reinterpret_cast<TreeSmem*>(treeRaw);
+    // (a following launch with programmatic serialization may start once every CTA of this grid runs)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t warp = threadIdx.x >> 5, lane = laneId();
+    const uint32_t huge = a.huge(), big = a.big();
+    auto viewOf = [&](uint32_t gt) -> const ViewDev& { return viewOfBlock(a.views, a.blockView, a.viewCount, gt / kTilesPerBlock); };
+    auto ctaTile = [&](uint32_t gt) {
+        const ViewDev& V = viewOf(gt);
+        const uint32_t tile = gt - V.tileStart;
+        bool overflow;
+        const uint32_t visits = treeTile<kTreeWarps>(a, V, tile, sm.head[0], sm.cta, overflow);
+        if (threadIdx.x == 0) {
+            V.tileCost[tile] = visits;
+            if (overflow) {
+                V.tileLists[tile] = TileList{kNoChunk, 0};
+                a.retry[a.first + atomicAdd(a.retryCount, 1u)] = gt;
+            }
+        }
+        publishTile<kTreeWarps>(a, gt, overflow);
+    };
+    if (threadIdx.x == 0) sm.spill = kNoChunk;
+    bool tookBig = false;
+    for (;;) {
+        if (threadIdx.x == 0) sm.item = huge + atomicAdd(a.bigQueue, 1u);
+        __syncthreads();
+        const uint32_t w = sm.item;
+        __syncthreads();
+        if (w >= big) break;
+        tookBig = true;
+        ctaTile(a.order ? a.order[a.first + w] : a.first + w);
+        if (!a.persistent) break;
+    }
+    while (a.persistent || !tookBig) {
+        uint32_t w = 0;
+        if (lane == 0) w = atomicAdd(a.queue, 1u);
+        w = big + __shfl_sync(kFull, w, 0);
+        if (w >= a.count) break;
+        const uint32_t gt = a.order ? a.order[a.first + w] : a.first + w;
+        const ViewDev& V = viewOf(gt);
+        const uint32_t tile = gt - V.tileStart;
+        bool overflow;
+        const uint32_t visits = treeTile<1>(a, V, tile, sm.head[warp], sm.warp[warp], overflow);
+        if (overflow) {
+            if (lane == 0) V.tileLists[tile].first = atomicExch(&sm.spill, gt);
+        } else {
+            if (lane == 0) V.tileCost[tile] = visits;
+            publishTile<1>(a, gt, false);
+        }
+        __syncwarp();
+        if (!a.persistent) break;
+    }
+    __syncthreads();
+    for (uint32_t gt = sm.spill; gt != kNoChunk;) {
+        const ViewDev& V = viewOf(gt);
+        const uint32_t next = *reinterpret_cast<volatile uint32_t*>(&V.tileLists[gt - V.tileStart].first);
+        __syncthreads();
+        ctaTile(gt);
+        __syncthreads();
+        gt = next;
+    }
+    // this grid ends after the one that it started beside (tileTreeHugeKernel), so that a later launch
+    // finds both lists' tiles complete
+    if (blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The tiles that a whole SM's shared memory is for. LIST = false: the class's tiles that were this
+// large in the last frame, before its other tiles (a tile that still outgrows the store, or cannot be
+// culled breadth first, goes to the retry list). LIST = true: the retry list; what the store cannot
+// take, and every tile when tree is 0, is culled by one warp with the sequential traversal and the
+// reference's TileFrame capacity (4096 entries, 48 KiB).
+template <bool LIST>
+__global__ void __launch_bounds__(kHugeWarps * 32, 1) tileTreeHugeKernel(TileCullArgs a, uint32_t tree) {
+    extern __shared__ __align__(16) unsigned char treeRaw[];
+    HugeSmem& sm = *reinterpret_cast<HugeSmem*>(treeRaw);
+    if (!LIST) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t count = LIST ? *reinterpret_cast<volatile uint32_t*>(a.retryCount) : a.huge();
+    for (uint32_t w = blockIdx.x; w < count; w += gridDim.x) {
+        const uint32_t gt = LIST ? a.retry[a.first + w] : a.order[a.first + w];
+        const ViewDev& V = viewOfBlock(a.views, a.blockView, a.viewCount, gt / kTilesPerBlock);
+        const uint32_t tile = gt - V.tileStart;
+        bool overflow = true;
+        uint32_t visits = 0;
+        if (tree) {
+            visits = treeTile<kHugeWarps>(a, V, tile, sm.head, sm.cta, overflow);
+            __syncthreads();
+        }
+        if (LIST && overflow && threadIdx.x < 32) {
+            visits = cullTile(a, V, tile, sm.seq, overflow);
+            if (overflow && threadIdx.x == 0) atomicOr(&a.counters[1], kStatusStackOverflow);
+        }
+        if (threadIdx.x == 0) {
+            V.tileCost[tile] = visits;
+            if (!LIST && overflow) {
+                V.tileLists[tile] = TileList{kNoChunk, 0};
+                a.retry[a.first + atomicAdd(a.retryCount, 1u)] = gt;
+            }
+        }
+        if (!LIST) publishTile<kHugeWarps>(a, gt, overflow);
+        __syncthreads();
+    }
+}
+
+// Orders the global tiles by (rate class ascending, cost descending), cost in quarter octaves
+// of last frame's visit counts, and counts each class's large tiles (their buckets lie at the front
+// of the class). One block; positions within a bucket are in arrival order.
+constexpr uint32_t kCostBuckets = 132, kOrderBuckets = kRateClasses * kCostBuckets;
+constexpr uint32_t kOrderPerThread = (kOrderBuckets + 1023) / 1024;
+__host__ __device__ constexpr uint32_t costBucket(uint32_t c, uint32_t log2) { return kCostBuckets - 1 - (log2 * 4 + (((c + 1) << (31 - log2)) >> 29 & 3u)); }
+// A tile of at least kBigCost visits is culled by a whole CTA and one of at least kHugeCost by a CTA
+// with an SM's shared memory: bucket bounds that leave a warp's store (kWarpNodes) a third and a
+// CTA's (kCtaNodes) an eighth of headroom for a view that moves between frames (a huge tile holds a
+// whole SM: starting them at 1,536 visits took 6.0 ms instead of 2.8 for the cull of a foveated
+// frame with a thousand of them).
+constexpr uint32_t kBigCost = 191, kHugeCost = 1791;
+constexpr uint32_t kBigBuckets = costBucket(kBigCost, 7) + 1, kHugeBuckets = costBucket(kHugeCost, 10) + 1;
 __global__ void __launch_bounds__(1024) tileOrderKernel(FrameDev fr) {
-    __shared__ uint32_t hist[kOrderBuckets];
-    __shared__ uint32_t start[kOrderBuckets];
-    for (uint32_t b = threadIdx.x; b < kOrderBuckets; b += blockDim.x) hist[b] = 0;
+    __shared__ uint32_t hist[kOrderPerThread * 1024];
+    __shared__ uint32_t warpSum[32];
+    const uint32_t tid = threadIdx.x, lane = laneId();
+    for (uint32_t b = tid; b < kOrderPerThread * 1024; b += 1024) hist[b] = 0;
     __syncthreads();
     auto bucket = [&](uint32_t t) {
         const ViewDev& V = viewOfBlock(fr.views, fr.blockView, fr.viewCount, t / kTilesPerBlock);
-        const uint32_t c = V.tileCost[t - V.tileStart];
-        return V.rateIdx * 33u + uint32_t(__clz(c + 1u)); // clz falls as the cost grows
+        const uint32_t c = min(V.tileCost[t - V.tileStart], 0x7ffffffeu);
+        return V.rateIdx * kCostBuckets + costBucket(c, 31u - __clz(c + 1u));
     };
-    for (uint32_t t = threadIdx.x; t < fr.tiles; t += blockDim.x) atomicAdd(&hist[bucket(t)], 1u);
+    for (uint32_t t = tid; t < fr.tiles; t += 1024) atomicAdd(&hist[bucket(t)], 1u);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t b = 0; b < kOrderBuckets; b++) {
-            start[b] = run;
-            run += hist[b];
+    uint32_t mine[kOrderPerThread], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kOrderPerThread; k++) {
+        mine[k] = sum;
+        sum += hist[tid * kOrderPerThread + k];
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) warpSum[tid >> 5] = inc;
+    __syncthreads();
+    if (tid < 32) {
+        const uint32_t n = warpSum[lane];
+        uint32_t w = n;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, w, o);
+            if (lane >= o) w += y;
         }
+        warpSum[lane] = w - n;
     }
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < fr.tiles; t += blockDim.x) fr.order[atomicAdd(&start[bucket(t)], 1u)] = t;
+    const uint32_t base = warpSum[tid >> 5] + inc - sum;
+#pragma unroll
+    for (uint32_t k = 0; k < kOrderPerThread; k++) hist[tid * kOrderPerThread + k] = base + mine[k];
+    __syncthreads();
+    // (the exclusive prefix before the scatter moves it)
+    if (fr.bigCountOut && tid < 2 * kRateClasses) {
+        const uint32_t* h = hist + (tid >> 1) * kCostBuckets;
+        fr.bigCountOut[tid] = h[tid & 1u ? kHugeBuckets : kBigBuckets] - h[0];
+    }
+    __syncthreads();
+    for (uint32_t t = tid; t < fr.tiles; t += 1024) fr.order[atomicAdd(&hist[bucket(t)], 1u)] = t;
 }
 
 __global__ void writeViewKernel(ViewDev v, ViewDev* dst) { *dst = v; }
@@ -979,7 +1703,7 @@ __global__ void __launch_bounds__(1024) occupiedRankKernel(FrameDev fr) {
 struct DeviceLimits {
     int sms = 0;
     int ctasPerSm[9] = {};  // indexed by warps per CTA
-    bool retryReady = false;
+    bool treeReady = false;
 };
 
 // per-device launch limits, filled on first use; host threads rendering on different streams
@@ -1022,21 +1746,49 @@ cudaError_t launchTileCullW(const TileCullArgs& a, uint32_t count, uint32_t capP
     return cudaGetLastError();
 }
 
-// the retry pass: one warp per CTA, one CTA per SM; it reads the retry count on the device and
-// exits at once when no tile overflowed
-cudaError_t launchTileCullRetry(const TileCullArgs& a, cudaStream_t st) {
+// shared-memory sizes above the default, set once per device
+cudaError_t treeReady(DeviceLimits& d) {
+    std::lock_guard<std::mutex> lock(gLimitsMutex);
+    if (d.treeReady) return cudaSuccess;
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(tileTreeKernel, at, int(sizeof(TreeSmem)));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(tileTreeHugeKernel<false>, at, int(sizeof(HugeSmem)));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(tileTreeHugeKernel<true>, at, int(sizeof(HugeSmem)));
+    d.treeReady = e == cudaSuccess;
+    return e;
+}
+
+cudaError_t launchTileTree(const TileCullArgs& a, uint32_t capPerSm, cudaStream_t st) {
     DeviceLimits& d = limits();
-    const size_t smem = sizeof(TileSmemT<kRetryStack>);
-    {
-        std::lock_guard<std::mutex> lock(gLimitsMutex);
-        if (!d.retryReady) {
-            const cudaError_t e =
-                cudaFuncSetAttribute(tileCullRetryKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            d.retryReady = true;
-        }
+    cudaError_t e = treeReady(d);
+    if (e != cudaSuccess) return e;
+    // (how many tiles are large is known on the device only, so a CTA per tile, up to what is resident)
+    const uint32_t resident = uint32_t(d.sms) * (capPerSm ? std::min(capPerSm, 4u) : 4u);
+    const uint32_t grid = a.persistent ? std::min(a.count, resident) : a.count;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kTreeWarps * 32);
+    cfg.dynamicSmemBytes = sizeof(TreeSmem);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (a.counts) {
+        tileTreeHugeKernel<false><<<std::min<uint32_t>(a.count, d.sms), kHugeWarps * 32, sizeof(HugeSmem), st>>>(a, 1u);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        // the other tiles' cull starts beside it, once its CTAs run
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
     }
-    tileCullRetryKernel<<<d.sms, 32, smem, st>>>(a);
+    return cudaLaunchKernelEx(&cfg, tileTreeKernel, a);
+}
+
+// the retry pass: it reads the retry count on the device and exits at once when the list is empty
+cudaError_t launchTileCullRetry(const TileCullArgs& a, bool tree, cudaStream_t st) {
+    DeviceLimits& d = limits();
+    const cudaError_t e = treeReady(d);
+    if (e != cudaSuccess) return e;
+    tileTreeHugeKernel<true><<<std::min<uint32_t>(a.count, d.sms), kHugeWarps * 32, sizeof(HugeSmem), st>>>(a, tree ? 1u : 0u);
     return cudaGetLastError();
 }
 
@@ -1058,11 +1810,17 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
                                uint32_t* queues, uint32_t warps, uint32_t stackLimit, uint32_t* ready,
                                uint32_t* readyTail, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
-    if (stackLimit == 0 || stackLimit > kTileStack) stackLimit = kTileStack;
+    if (stackLimit == 0) {
+        const TileCullArgs t{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
+                             order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, ready, readyTail,
+                             fr.cullPersistent ? 1u : 0u, 0u, order ? fr.bigCount : nullptr, fr.bigSkip, queues + 3};
+        return launchTileTree(t, fr.cullCtasPerSm, st);
+    }
+    if (stackLimit > kTileStack) stackLimit = kTileStack;
     if (stackLimit < 8) return cudaErrorInvalidValue;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, queues + 2, stackLimit, ready, readyTail,
-                         fr.cullPersistent ? 1u : 0u, ready ? fr.streamTiles : 0u};
+                         fr.cullPersistent ? 1u : 0u, ready ? fr.streamTiles : 0u, nullptr, 0u, nullptr};
     switch (warps) {
     case 1: return launchTileCullW<1>(a, count, fr.cullCtasPerSm, st);
     case 2: return launchTileCullW<2>(a, count, fr.cullCtasPerSm, st);
@@ -1073,19 +1831,19 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
 }
 
 cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
-                                    uint32_t* queues, cudaStream_t st) {
+                                    uint32_t* queues, uint32_t stackLimit, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, nullptr, nullptr, 1u,
-                         0u};
-    return launchTileCullRetry(a, st);
+                         0u, nullptr, 0u, nullptr};
+    return launchTileCullRetry(a, stackLimit == 0, st);
 }
 
 cudaError_t launchTileCull(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
                            uint32_t* queues, uint32_t warps, uint32_t stackLimit, cudaStream_t st) {
     const cudaError_t e = launchTileCullMain(fr, order, first, count, queues, warps, stackLimit, nullptr, nullptr, st);
     if (e != cudaSuccess) return e;
-    return launchTileCullRetryPass(fr, order, first, count, queues, st);
+    return launchTileCullRetryPass(fr, order, first, count, queues, stackLimit, st);
 }
 
 cudaError_t launchOccupiedRank(const FrameDev& fr, cudaStream_t st) {

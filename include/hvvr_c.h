@@ -414,20 +414,25 @@ int hvvr_polar_foveated_samples(const hvvr_spec* spec, float* beams9, uint32_t* 
  * that rendered it last. Destroy batches before their raycasters; a batch whose raycaster
  * was destroyed returns HVVR_ERR_STATE. */
 typedef struct {
-    uint32_t tile_cull_warps;     /* warps per CTA of the tile-cull work queue: 1 (default), 2, 4 or 8 */
-    uint32_t heavy_divisor;       /* 1/heavy_divisor of each rate's tiles (last frame's slowest) are
-                                     culled and shaded on their own stream; 0 = no split */
+    uint32_t tile_cull_warps;     /* warps per CTA of the sequential tile cull's work queue (tile_stack_entries):
+                                     1 (default), 2, 4 or 8 */
+    uint32_t heavy_divisor;       /* with the sequential tile cull: 1/heavy_divisor of each rate's tiles (last
+                                     frame's slowest) are culled and shaded on their own stream; 0 = no split */
     uint64_t tri_index_capacity;  /* triangle-list pool entries shared by all views */
     uint32_t use_graph;           /* replay frames from a CUDA graph once the layout is stable */
     float frame_ms;               /* autotune result: median device time of a frame */
-    uint32_t tile_stack_entries;  /* traversal stack of the main tile-cull pass, 0 (= 256) or 8..256;
-                                     tiles that need more are culled again with 4096 entries */
+    uint32_t tile_stack_entries;  /* 0 (default): tiles are culled breadth first, what does not fit with the
+                                     reference's 4096-entry stack. 8..256: every tile is culled node by node
+                                     with a stack of this size; tiles that need more are culled again with
+                                     4096 entries. The lists are the same */
     uint32_t timing;              /* 1: record per-stage and per-launch events (the stage, kernel and
                                      part read-backs); they cost device time (about 0.4 ms of a 6 ms
                                      stereo frame). 0 (default): the frame's start and end only */
     uint32_t pipeline;            /* 1 (default): each part of a pinhole rate class runs its tile cull
                                      and its intersect/shade as one pipeline - a tile is shaded as soon
-                                     as its list is complete, while other tiles are still being culled.
+                                     as its list is complete, while other tiles are still being culled
+                                     (from 16 subsamples only with tile_stack_entries: the cull is then
+                                     a small part of the class).
                                      0: the cull of a part finishes before its intersect/shade starts */
     uint32_t tile_cull_ctas_per_sm; /* cap on the persistent tile cull's resident CTAs per SM (0 = as many
                                      as fit): leaves room on every SM for other work (the intersect of
