@@ -613,12 +613,11 @@ int cloneCamera(const hvvr_camera* src, hvvr_camera** out) {
 constexpr uint32_t kSplitMinTiles = 32;
 
 void batchConfigDefault(hvvr_batch_config* c) {
-    // On the 1M-triangle stereo 2x1080x1200 8xMSAA frame, one-warp cull CTAs with the slowest 1/8
+    // The sequential cull's settings, on the 1M-triangle stereo 2x1080x1200 8xMSAA frame: one-warp cull CTAs with the slowest 1/8
     // of the tiles as the heavy part, cull -> shade pipeline on, were fastest: 4.92 ms against 5.50
     // with 2-warp CTAs (a warp that runs out of tiles frees its registers for the shade of finished
     // tiles at once); heavy shares 1/4, 1/6, 1/12 and 1/16 were 5.17, 5.05, 5.19 and 5.3-5.4 ms;
-    // without the pipeline 5.99. Streaming the lists of the first 400 tiles of each rate class's first
-    // part: 4.86 ms against 4.99 without (16, 48, 148, 1000, 2544 tiles: 4.99, 4.99, 4.89, 4.87, 5.00)
+    // without the pipeline 5.99.
     c->tile_cull_warps = 1;
     c->heavy_divisor = 8;
     c->tri_index_capacity = kDefaultCapacity;
@@ -790,7 +789,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     for (auto& u : b->kevUsed) u = false;
     for (auto& u : b->kevPipelined) u = false;
     // the frame as the tile cull of class r sees it, `skip` tiles into the class
-    auto part1 = [](const FrameDev& f, uint32_t r, uint32_t skip) {
+    auto ofClass = [](const FrameDev& f, uint32_t r, uint32_t skip) {
         FrameDev p = f;
         p.bigCount = f.counters + kBigBase + 2 * r;
         p.bigSkip = skip;
@@ -817,10 +816,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             // CTAs are better used from the cull's end, longest tile first, than waiting for tiles.
             const bool piped = b->cfg.pipeline && (msaa < 16 || b->cfg.tile_stack_entries);
             if (!lens && piped) {
-                // the class's first part holds its longest tiles: those stream their lists
-                FrameDev fp = part1(fr, r, p0 - rs);
-                fp.streamTiles = part == (heavy ? 0u : 1u) ? b->cfg.stream_tiles : 0u;
-                CUDA_TRY(launchCullShadePipeline(fp, msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
+                CUDA_TRY(launchCullShadePipeline(ofClass(fr, r, p0 - rs), msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                                  fr.counters + kPipeBase + k, b->cfg.tile_cull_warps,
                                                  b->cfg.tile_stack_entries, ps));
                 // the cull and the shade overlap: one event marks the end of both (and of the retry
@@ -836,7 +832,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
                 CUDA_TRY(cudaStreamWaitEvent(st, b->doneEv[k], 0));
                 continue;
             }
-            CUDA_TRY(launchTileCull(part1(fr, r, p0 - rs), fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
+            CUDA_TRY(launchTileCull(ofClass(fr, r, p0 - rs), fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                     b->cfg.tile_cull_warps, b->cfg.tile_stack_entries, ps));
             if (stages) CUDA_TRY(recordStage(b->kev[k][1], ps, capturing));
             if (stages && part == 1 && first) CUDA_TRY(recordStage(b->ev[2], ps, capturing));
@@ -1117,8 +1113,7 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
         std::vector<uint64_t> gkey = b->layoutKey;
         const uint64_t extra[] = {b->cfg.tile_cull_warps, b->cfg.heavy_divisor, b->poolChunks, strict ? 1u : 0u,
                                   uint64_t(uintptr_t(st)), b->cfg.tile_stack_entries, b->cfg.timing,
-                                  b->cfg.pipeline, b->cfg.tile_cull_ctas_per_sm, b->cfg.tile_cull_persistent,
-                                  b->cfg.stream_tiles};
+                                  b->cfg.pipeline, b->cfg.tile_cull_ctas_per_sm, b->cfg.tile_cull_persistent};
         gkey.insert(gkey.end(), std::begin(extra), std::end(extra));
         if (!b->graph || gkey != b->graphKey) {
             dropGraph(b);

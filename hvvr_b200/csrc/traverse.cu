@@ -462,15 +462,6 @@ struct TileSmemT {
     uint32_t rStart[kRanges], rLen[kRanges];
 };
 
-// End of a streamed tile's list: every lane's list writes are visible device-wide before lane 0
-// releases the last chunk's link as kNoChunk.
-__device__ __forceinline__ void endStream(uint32_t* lastLink) {
-    __threadfence();
-    __syncwarp();
-    if (laneId() == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(lastLink), "r"(kNoChunk) : "memory");
-    __syncwarp();
-}
-
 struct Emitter {
     uint32_t* pool;
     uint32_t* chunkNext;
@@ -479,16 +470,8 @@ struct Emitter {
     uint32_t first, prev, bufCount, stored, total;
     bool dead;
     uint32_t rc; // ranges buffered in rStart/rLen
-    // streamed tile (stream): published with its first chunk; list = its TileList, ready = the
-    // launch's ready slots, gt = the global tile index the slot carries
-    bool stream, published;
-    TileList* list;
-    uint32_t* ready;
-    uint32_t* readyTail;
-    uint32_t gt;
 
-    // last: the list's final (partial) chunk
-    __device__ void flush(uint32_t* buf, bool last = false) {
+    __device__ void flush(uint32_t* buf) {
         __syncwarp();
         uint32_t c = 0;
         if (laneId() == 0) c = atomicAdd(&counters[0], 1u);
@@ -500,27 +483,7 @@ struct Emitter {
         }
         const uint4 w = reinterpret_cast<const uint4*>(buf)[laneId()];
         reinterpret_cast<uint4*>(pool + size_t(c) * kChunk)[laneId()] = w;
-        if (stream && (prev != kNoChunk || !last)) {
-            // The chunk's entries and its pending link are visible device-wide before the chunk is
-            // linked to its predecessor, or, the first chunk, before the tile is published with a
-            // streaming TileList. (A list that fits one chunk is published at the end as usual.)
-            if (laneId() == 0) chunkNext[c] = kChunkPending;
-            __threadfence();
-            __syncwarp();
-            if (laneId() == 0) {
-                if (prev != kNoChunk) {
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(chunkNext + prev), "r"(c) : "memory");
-                } else {
-                    *list = TileList{c, kCountStreaming};
-                    __threadfence();
-                    const uint32_t pos = atomicAdd(readyTail, 1u);
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ready + pos), "r"(gt) : "memory");
-                }
-            }
-            if (prev == kNoChunk) published = true;
-        } else if (laneId() == 0) {
-            if (prev != kNoChunk) chunkNext[prev] = c;
-        }
+        if (laneId() == 0 && prev != kNoChunk) chunkNext[prev] = c;
         if (prev == kNoChunk) first = c;
         prev = c;
         stored += bufCount;
@@ -614,7 +577,6 @@ struct TileCullArgs {
     uint32_t* ready;       // pipelined: ready slots, slot first + i for the i-th finished tile (else nullptr)
     uint32_t* readyTail;   // pipelined: finished tiles so far, zero at launch
     uint32_t persistent;   // 0: every warp culls one tile (the grid has a warp per tile), then exits
-    uint32_t streamTiles;  // with ready: queue positions below this stream their lists (else 0)
     const uint32_t* counts; // breadth-first cull: the large, and of those the huge, tiles at the front of the rate
                            // class's order (nullptr: none)
     uint32_t skip;         // tiles of the class before `first`
@@ -628,8 +590,7 @@ struct TileCullArgs {
 // traverseTiles for one tile of view V (tile = view-local index); returns the node visits.
 // overflow: the sorted stack needed more than S entries; the tile's list is left empty.
 template <uint32_t S>
-__device__ uint32_t cullTile(const TileCullArgs& a, const ViewDev& V, uint32_t tile, TileSmemT<S>& s,
-                             bool& overflow, bool stream = false, uint32_t gt = 0, bool* published = nullptr) {
+__device__ uint32_t cullTile(const TileCullArgs& a, const ViewDev& V, uint32_t tile, TileSmemT<S>& s, bool& overflow) {
     overflow = false;
     const uint32_t lane = laneId();
     const Node* __restrict__ nodes = V.nodes;
@@ -653,9 +614,7 @@ __device__ uint32_t cullTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
     __syncwarp();
     const LaneTest t = loadLaneTest(s.f);
     const int distIdx = s.f.distIdx;
-    Emitter em{a.pool, a.chunkNext, a.poolChunks, a.counters, kNoChunk, kNoChunk, 0, 0, 0, false, 0,
-               stream && a.ready != nullptr, false, V.tileLists + tile, a.ready ? a.ready + a.first : nullptr,
-               a.readyTail, gt};
+    Emitter em{a.pool, a.chunkNext, a.poolChunks, a.counters, kNoChunk, kNoChunk, 0, 0, 0, false, 0};
     uint32_t top = stackSize - 1;
     uint32_t node = s.node[top];
     uint32_t visits = 0;
@@ -826,32 +785,12 @@ __device__ uint32_t cullTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
     vcLast = phaseClock(top);
 #endif
     if (overflow) {
-        // (a streamed tile's shade ends its chunk walk here; the retry passes cull and shade the
-        // tile again after it)
-        if (published) *published = em.published;
-        if (em.published) endStream(a.chunkNext + em.prev);
         if (lane == 0) V.tileLists[tile] = TileList{kNoChunk, 0};
         return visits;
     }
     if (!em.dead && em.rc) em.expand(s);
-    if (em.published && !em.dead && em.bufCount) {
-        // a streamed list's last chunk: its unused entries say so
-        for (uint32_t i = em.bufCount + lane; i < kChunk; i += 32) s.buf[i] = kNoTriangle;
-        __syncwarp();
-    }
-    if (!em.dead && em.bufCount) em.flush(s.buf, true);
-    // (after the last expansion, whose full chunks may have published the tile)
-    if (published) *published = em.published;
-    if (em.published) {
-        // the last chunk's end-of-list link, then the complete TileList, each after what precedes it
-        endStream(a.chunkNext + em.prev);
-        if (lane == 0) {
-            __threadfence();
-            const unsigned long long l =
-                uint64_t(em.first) | (uint64_t(em.dead ? em.stored : em.total) << 32);
-            asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(V.tileLists + tile), "l"(l) : "memory");
-        }
-    } else if (lane == 0) {
+    if (!em.dead && em.bufCount) em.flush(s.buf);
+    if (lane == 0) {
         if (em.prev != kNoChunk) a.chunkNext[em.prev] = kNoChunk;
         V.tileLists[tile] = TileList{em.first, em.dead ? em.stored : em.total};
     }
@@ -863,6 +802,21 @@ __device__ uint32_t cullTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
     }
 #endif
     return visits;
+}
+
+// Publishes a finished tile to the concurrent shade: every thread's list writes are made visible
+// device-wide before one releases the ready slot.
+template <int W>
+__device__ __forceinline__ void publishTile(const TileCullArgs& a, uint32_t gt, bool retry) {
+    if (!a.ready) return;
+    __threadfence();
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+    if ((W == 1 ? laneId() : threadIdx.x) == 0) {
+        const uint32_t pos = atomicAdd(a.readyTail, 1u);
+        const uint32_t val = gt | (retry ? kReadyRetry : 0u);
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.ready + a.first + pos), "r"(val) : "memory");
+    }
 }
 
 // Persistent warps pull tiles from a queue (longest-first when an order is given), so a
@@ -889,23 +843,13 @@ __global__ void __launch_bounds__(W * 32, W == 1 ? 20 : 1) tileCullKernel(TileCu
         const ViewDev& V = viewOfBlock(a.views, a.blockView, a.viewCount, gt / kTilesPerBlock);
         const uint32_t tile = gt - V.tileStart;
         __syncwarp();
-        bool overflow, published = false;
-        const uint32_t visits = cullTile(a, V, tile, s, overflow, w < a.streamTiles, gt, &published);
+        bool overflow;
+        const uint32_t visits = cullTile(a, V, tile, s, overflow);
         if (lane == 0) {
             V.tileCost[tile] = visits;
             if (overflow) a.retry[a.first + atomicAdd(a.retryCount, 1u)] = gt;
         }
-        if (a.ready && !published) {
-            // publish: every lane's list writes (pool chunks, links, the tile's TileList) are made
-            // visible device-wide before lane 0 releases the slot
-            __threadfence();
-            __syncwarp();
-            if (lane == 0) {
-                const uint32_t pos = atomicAdd(a.readyTail, 1u);
-                const uint32_t val = gt | (overflow ? kReadyRetry : 0u);
-                asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.ready + a.first + pos), "r"(val) : "memory");
-            }
-        }
+        publishTile<1>(a, gt, overflow);
         __syncwarp();
         if (!a.persistent) return;
     }
@@ -1478,21 +1422,6 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
     return visits;
 }
 
-// Publishes a finished tile to the concurrent shade: every thread's list writes are made visible
-// device-wide before one releases the ready slot.
-template <int W>
-__device__ __forceinline__ void publishTile(const TileCullArgs& a, uint32_t gt, bool retry) {
-    if (!a.ready) return;
-    __threadfence();
-    if constexpr (W == 1) __syncwarp();
-    else __syncthreads();
-    if ((W == 1 ? laneId() : threadIdx.x) == 0) {
-        const uint32_t pos = atomicAdd(a.readyTail, 1u);
-        const uint32_t val = gt | (retry ? kReadyRetry : 0u);
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.ready + a.first + pos), "r"(val) : "memory");
-    }
-}
-
 // Persistent CTAs. The tiles that were large in the last frame (a.counts[0] tiles at the front of the
 // class's order, of which the first a.counts[1] are culled by tileTreeHugeKernel) are culled by a whole
 // CTA each, then every warp takes small ones; a small one that outgrows its warp's store is kept in a
@@ -1813,14 +1742,14 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
     if (stackLimit == 0) {
         const TileCullArgs t{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                              order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, ready, readyTail,
-                             fr.cullPersistent ? 1u : 0u, 0u, order ? fr.bigCount : nullptr, fr.bigSkip, queues + 3};
+                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.bigSkip, queues + 3};
         return launchTileTree(t, fr.cullCtasPerSm, st);
     }
     if (stackLimit > kTileStack) stackLimit = kTileStack;
     if (stackLimit < 8) return cudaErrorInvalidValue;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, queues + 2, stackLimit, ready, readyTail,
-                         fr.cullPersistent ? 1u : 0u, ready ? fr.streamTiles : 0u, nullptr, 0u, nullptr};
+                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, nullptr};
     switch (warps) {
     case 1: return launchTileCullW<1>(a, count, fr.cullCtasPerSm, st);
     case 2: return launchTileCullW<2>(a, count, fr.cullCtasPerSm, st);
@@ -1835,7 +1764,7 @@ cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, u
     if (count == 0) return cudaSuccess;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, nullptr, nullptr, 1u,
-                         0u, nullptr, 0u, nullptr};
+                         nullptr, 0u, nullptr};
     return launchTileCullRetry(a, stackLimit == 0, st);
 }
 
