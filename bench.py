@@ -202,7 +202,8 @@ def frame_counts(hv, scenes, sc):
     rc.render()
     ctr = rc.counters()
     out = {"padded_samples": 0, "tiles": 0, "list_entries": 0, "unique_hits": 0, "node_visits": 0,
-           "tested_entries": int(ctr[4]), "tested_warp_entries": int(ctr[5]), "longest_tile_node_visits": 0}
+           "tested_entries": int(ctr[4]), "tested_warp_entries": int(ctr[5]), "tested_sample_entries": int(ctr[6]),
+           "longest_tile_node_visits": 0}
     for cam in cams:
         blocks, tiles, padded, msaa = cam.layout()
         n, tri, mask = cam.gbuffer()
@@ -225,11 +226,11 @@ def intersect_bytes(c):
 
 
 def intersect_flops(c, msaa):
-    """FP32 operations of a frame's executed intersect tests: every (warp of 32 samples, surviving
-    list entry) pair whose tests ran (counted on the device; pairs the per-warp depth bound skips are
-    not counted), 72 flops of per-(sample, triangle) setup (IntersectTriangleThread +
-    GetDifferentials) and 16 per subsample test (7 FMA + 2 adds) per sample."""
-    return c["tested_warp_entries"] * 32 * (72 + 16 * msaa)
+    """FP32 operations of a frame's executed intersect tests: every (sample, list entry) pair whose
+    tests ran (counted on the device; the pairs that the footprint and depth bounds pass by are not
+    counted, nor are the bounds themselves), 72 flops of per-(sample, triangle) setup
+    (IntersectTriangleThread + GetDifferentials) and 16 per subsample test (7 FMA + 2 adds)."""
+    return c["tested_sample_entries"] * (72 + 16 * msaa)
 
 
 def fp32_line(c, msaa, launch_ms, sm_mhz):
@@ -1012,7 +1013,8 @@ def run_foveated(args):
     rc.render()
     ctr = rc.counters()
     counts = {"padded_samples": 0, "tiles": 0, "list_entries": 0, "unique_hits": 0, "node_visits": 0,
-              "tested_entries": int(ctr[4]), "tested_warp_entries": int(ctr[5])}
+              "tested_entries": int(ctr[4]), "tested_warp_entries": int(ctr[5]),
+              "tested_sample_entries": int(ctr[6])}
     for cam in cams:
         blocks, tiles, padded, msaa = cam.layout()
         n, tri, mask = cam.gbuffer()

@@ -698,9 +698,10 @@ class Raycaster:
 
     def counters(self):
         """the last frame's counters: list pool entries, retried tiles, status, views, list entries
-        that passed the intersect's per-tile tests, (warp, entry) pairs whose subsample tests ran"""
-        t = np.zeros(6, dtype=np.uint64)
-        _check(_lib.hvvr_raycaster_read_counters(self.handle, t.ctypes.data, 6))
+        that passed the intersect's per-tile tests, (warp, entry) and (sample, entry) pairs whose
+        subsample tests ran"""
+        t = np.zeros(7, dtype=np.uint64)
+        _check(_lib.hvvr_raycaster_read_counters(self.handle, t.ctypes.data, 7))
         return t
 
     def part_times(self):

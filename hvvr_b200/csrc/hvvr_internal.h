@@ -218,15 +218,16 @@ enum : uint32_t { kRateClasses = 18 };
 // counters: [0] chunk allocator, [1] status, then per tile-cull launch k (2 per rate class)
 // four words at kQueueBase + 4k: work-queue head, retry count, retry-queue head, large tiles' queue head
 // then one word counting the list entries that survive the intersect's per-tile tests, one counting
-// the (warp, surviving entry) pairs whose subsample tests ran (the rest were skipped by the per-warp
-// depth bound), then per launch part k (2 per rate class) the ready-slot tail of its cull -> shade
-// pipeline
+// the (warp, surviving entry) pairs of which some sample's subsample tests ran, one counting the
+// (sample, surviving entry) pairs whose subsample tests ran, then per launch part k (2 per rate class)
+// the ready-slot tail of its cull -> shade pipeline
 enum : uint32_t {
     kQueueBase = 2,
     kQueueWords = 4,
     kSurvivorWord = kQueueBase + kQueueWords * 2 * kRateClasses,
     kTestedWord = kSurvivorWord + 1,
-    kPipeBase = kTestedWord + 1,
+    kSampleTestedWord = kTestedWord + 1,
+    kPipeBase = kSampleTestedWord + 1,
     kBigBase = kPipeBase + 2 * kRateClasses, // per rate class: its large and its huge tiles (tileOrderKernel)
     kCounterWords = kBigBase + 2 * kRateClasses
 };

@@ -1416,9 +1416,10 @@ static int frameCounters(const hvvr_batch* b, uint64_t* out, uint32_t count) {
     CUDA_TRY(cudaEventSynchronize(b->ev[5]));
     uint64_t retried = 0;
     for (uint32_t k = 0; k < 2 * kRateClasses; k++) retried += b->hostCounters[kQueueBase + kQueueWords * k + 1];
-    const uint64_t v[6] = {uint64_t(std::min(b->hostCounters[0], b->poolChunks)) * kChunk, retried, b->hostCounters[1],
-                           b->views.size(), b->hostCounters[kSurvivorWord], b->hostCounters[kTestedWord]};
-    for (uint32_t i = 0; i < count; i++) out[i] = i < 6 ? v[i] : 0u;
+    const uint64_t v[7] = {uint64_t(std::min(b->hostCounters[0], b->poolChunks)) * kChunk, retried, b->hostCounters[1],
+                           b->views.size(), b->hostCounters[kSurvivorWord], b->hostCounters[kTestedWord],
+                           b->hostCounters[kSampleTestedWord]};
+    for (uint32_t i = 0; i < count; i++) out[i] = i < 7 ? v[i] : 0u;
     return HVVR_OK;
 }
 

@@ -7,12 +7,13 @@
 // EmitGBuffer does (intersect.cu:28-89), and are shaded and resolved in the same thread
 // (ShadeMSAA, resolve.cu:161-284). The G-buffer therefore never goes to HBM.
 //
-// The tile's triangle list is consumed in its chunks of 128 entries. Each thread tests one
-// entry against the tile frustum planes, the ray-origin half space and the corner-ray
-// barycentric bounds (FrustumPlanes::test, IntersectTriangleTile<false>::setup,
-// TestTriangleFrustaUVW; libraries/hvvr/raycaster/prim_tests.h:18-164); survivors are compacted
-// into shared memory in list order with warp ballots, and every thread then tests its
-// sample's N subsamples against them in that order, so depth ties resolve as in the reference.
+// The tile's triangle list is consumed in chunks of 128 entries. The tile's own tests (frustum planes,
+// ray-origin half space, corner-ray barycentrics: FrustumPlanes::test, IntersectTriangleTile<false>::setup,
+// TestTriangleFrustaUVW; libraries/hvvr/raycaster/prim_tests.h:18-164) decide which triangles its
+// samples are tested against, and each sample takes those in list order, so depth ties resolve as in
+// the reference. Before and between them, bounds that no rounding can break (edgePlane) pass by what
+// a tile, a warp of its samples, or one sample cannot hit: a sample runs its N subsample tests on the
+// few triangles that its footprint meets in front of what it has already found, not on its tile's.
 #include <algorithm>
 
 #include "../../include/hvvr_c.h"
@@ -489,21 +490,42 @@ __device__ __forceinline__ bool uvwAllOut(const float (&ro)[4][3], const float (
     return uMax < 0 || uMin > 1 || vMax < 0 || vMin > 1 || wMax < 0 || wMin > 1;
 }
 
+// FrustumPlanes::test (prim_tests.h:30-50)
+__device__ __forceinline__ bool inFrustum(const float (&pl)[4][4], const TriGeom& tri) {
+    bool in = true;
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const F3 dir = f3(pl[p][0], pl[p][1], pl[p][2]);
+        const float dist = pl[p][3];
+        const float d0 = dot3(dir, tri.v0);
+        const float d1 = d0 + dot3(dir, tri.e0);
+        const float d2 = d0 + dot3(dir, tri.e1);
+        if (d0 > dist && d1 > dist && d2 > dist) in = false;
+    }
+    return in;
+}
+
+// The list is culled kBatchChunks chunks at a time; the next ones are copied in while their samples are tested.
+constexpr uint32_t kBatchChunks = 2, kBatchSlots = kBatchChunks * kChunk;
+
 struct ShadeSmem {
     float ro[4][3], rd[4][3]; // world corner rays
     float pl[4][4];           // frustum planes
-    // the chunk's surviving triangles, one array per component (a warp reads the same entry on
-    // every lane, and a pair of entries j, k loads straight into the two halves of a register
-    // pair): e0, e1, camPos - v0, e0 x e1, t, |e0 x e1| (the norm as computed in float, for the
-    // depth skip) and the triangle index
-    float g[12][kChunk];
-    float t[kChunk], nlen[kChunk];
-    uint32_t idx[kChunk];
-    uint32_t warpCount[4];
-    // the list triangles of the chunk being culled, 48 bytes per entry (three float4 rows of the
-    // triangle array), copied in by cp.async one chunk ahead; thread i writes and reads only
-    // entry i, so the copy of the next chunk can start as soon as entry i has been read
-    float4 stage[3 * kChunk];
+    uint16_t cand[kBatchSlots];     // slots (chunk of the batch * 128 + thread) of the entries that can meet the
+                                    // tile, in list order; they are tested kChunk at a time:
+    float4 edge[4][kChunk];         // their edge planes through the camera and normals, with slack (edgePlane),
+    float t[kChunk];
+    uint32_t idx[kChunk];           // t and triangle index,
+    uint32_t need[kChunk / 32][4];  // and per 32 of them and warp: which the warp's samples may hit
+    float dir[6][kTileSize];        // -du, -dv of every sample
+    float axis[3][4];          // three axes, about along the tile's beams' du, dv and c (orthonormal)
+    float4 box[3][5];          // along axis k, of warp 0-3's and (4) the whole tile's -c: middle, half extent
+    float warpT[4];            // per warp: the largest depth of its samples
+    float warpMax[2][4];       // per warp: the largest footprint radius and beam length
+    uint32_t warpCount[kBatchChunks][4];
+    // the list triangles, 48 bytes per entry (three float4 rows of the triangle array), copied in by
+    // cp.async
+    float4 tri[kBatchSlots][3];
 };
 
 // cp.async of 16 bytes, global to shared, cached in L2 only (the triangle rows are gathered once
@@ -515,10 +537,11 @@ __device__ __forceinline__ void cpAsync16(void* dst, const void* src) {
 __device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cpAsyncWaitAll() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// resident CTAs per SM the register allocation must allow (7 = 72 registers per thread)
-// resident CTAs per SM: N <= 8 at 72 registers; N = 16 at 96 (a few spilled bytes, 5.5% faster on
-// the 16xMSAA foveated frame than 4 CTAs at 107 registers without spills)
-template <uint32_t N> struct MinCtas { static constexpr int v = N <= 8 ? 7 : (N == 16 ? 5 : 4); };
+// resident CTAs per SM that the register allocation must allow. Launch alone, one B200: N = 8 (1M triangles,
+// stereo) 1,260 us with 7 CTAs of 72 registers, 1,305 with 8 of 64; N = 2 (1M, 1280 x 720) 484 and 565;
+// N = 16 (foveated) 2,450 us with 6 CTAs of 80 registers, 2,526 with 5 of 96; N = 32 863 us with 4 of
+// 128, 906 with 3 of 168.
+template <uint32_t N> struct MinCtas { static constexpr int v = N <= 8 ? 7 : (N == 16 ? 6 : 4); };
 
 // Where a shade launch takes its tiles from; item i of the launch is
 //   kFromOrder: order[first + i] (order == nullptr: first + i), i < count;
@@ -546,6 +569,90 @@ __device__ uint32_t waitReady(const uint32_t* slot, uint32_t* counters) {
         }
         __nanosleep(i < 32 ? 128 : 1024);
     }
+}
+
+// Most of a tile's list never meets a given sample: it lies beside it, or behind what the sample has
+// found. Testing every warp's 32 samples against every triangle that passed the tile's tests took
+// 14.9M (warp, triangle) pairs of N tests on the 1M-triangle stereo frame; with the bounds below 6.6M
+// (sample, triangle) pairs are left, tested two at a time. Launch alone, before and after: 1M triangles
+// stereo N = 8 3,253 and 1,260 us, 1280 x 720 N = 2 1,313 and 484, 500k 1280 x 720 N = 32 3,857 and 863, foveated N = 16
+// 7,941 and 2,450, 57k 640 x 480 N = 1 142 and 130. What bounds it now: issue (0.5 of the slots) and the
+// latency of the chain list entry - tile - warp - sample - test.
+//
+// Which samples can a triangle hit at all? A subsample's v, w and u are linear in its direction dir =
+// c + ax du + ay dv: v = -dir . gv with gv = v0r x e1, w = -dir . gw with gw = e0 x v0r, and u =
+// -dir . gu with gu = n - gv - gw. Each has to have its sign bit clear, so a sample is passed by
+// when for one of the three -c . g + radius |g| + (rounding) < 0, radius bounding |ax du + ay dv| (the
+// unit offsets lie in the unit disk). The rounding term covers what the test's own operations and
+// these may be off by: S = |v0r| (|e0| + |e1|) + |n| bounds every partial result over |dir|, each of
+// the two sides loses less than 45 half-ulps of S |dir|, and flushed denormals less than the last term.
+// The test also rejects a subsample when depth * denom < t: with denom = -dir . n at most d = -c . n +
+// radius |n| + (rounding), and no subsample's depth above T, t > T d passes the sample by (with d < 0
+// no subsample sees the front; the product's rounding is inside the slack).
+// The samples that are left are tested as before, so hits and depths are the same bits.
+// edge[e] = {g, slack}: -c . g + slack < 0 passes the sample by. (NaN keeps it.)
+__device__ __forceinline__ float4 edgePlane(F3 g, float radius, float slack) {
+    const float g2 = fmaxf(fmaf(g.x, g.x, fmaf(g.y, g.y, g.z * g.z)), 1e-30f);
+    float len;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(len) : "f"(g2));
+    return make_float4(g.x, g.y, g.z, fmaf(radius * 1.00001f, len, slack));
+}
+__device__ __forceinline__ float norm1(F3 v) { return (fabsf(v.x) + fabsf(v.y)) + fabsf(v.z); }
+__device__ __forceinline__ F3 cross3fma(F3 a, F3 b) {
+    return f3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
+}
+__device__ __forceinline__ float edgeValue(F3 nc, float4 e) { return fmaf(nc.x, e.x, fmaf(nc.y, e.y, fmaf(nc.z, e.z, e.w))); }
+// a plane's components along the tile's axes, and its value over a box of beams (its largest)
+__device__ __forceinline__ F3 edgeAlong(const ShadeSmem& sm, float4 e) {
+    const F3 g = f3(e.x, e.y, e.z);
+    float a[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) a[k] = fmaf(sm.axis[k][0], g.x, fmaf(sm.axis[k][1], g.y, sm.axis[k][2] * g.z));
+    return f3(a[0], a[1], a[2]);
+}
+__device__ __forceinline__ float edgeValue(const ShadeSmem& sm, uint32_t box, F3 a, float slack) {
+    const float2 x = *reinterpret_cast<const float2*>(&sm.box[0][box]), y = *reinterpret_cast<const float2*>(&sm.box[1][box]),
+                 z = *reinterpret_cast<const float2*>(&sm.box[2][box]);
+    return fmaf(x.x, a.x, fmaf(y.x, a.y, fmaf(z.x, a.z, fmaf(x.y, fabsf(a.x), fmaf(y.y, fabsf(a.y), fmaf(z.y, fabsf(a.z), slack))))));
+}
+// a triangle's planes: gv, gw, gu and the normal, and its t
+struct TriPlanes {
+    float4 e[4];
+    float t;
+};
+__device__ __forceinline__ TriPlanes trianglePlanes(const TriGeom& tri, F3 camPos, float radius, float maxLen) {
+    TriPlanes x;
+    const F3 nrm = cross3(tri.e0, tri.e1), v0r = camPos - tri.v0;
+    x.t = dot3(v0r, nrm);
+    const F3 gv = cross3fma(v0r, tri.e1), gw = cross3fma(tri.e0, v0r), gu = (nrm - gv) - gw;
+    const float s1 = norm1(tri.e0) + norm1(tri.e1);
+    const float slack = maxLen * (6e-6f * (norm1(v0r) * s1 + norm1(nrm)) + 1e-33f * (1.0f + s1));
+    x.e[0] = edgePlane(gv, radius, slack);
+    x.e[1] = edgePlane(gw, radius, slack);
+    x.e[2] = edgePlane(gu, radius, slack);
+    x.e[3] = edgePlane(nrm, radius, slack);
+    return x;
+}
+// whether some sample of a box (depths at most farT) may be hit; a0-a3 the planes along the axes
+__device__ __forceinline__ bool planesMeet(const ShadeSmem& sm, uint32_t box, F3 a0, F3 a1, F3 a2, F3 a3, const TriPlanes& x, float farT) {
+    const float lowest = fminf(edgeValue(sm, box, a0, x.e[0].w), fminf(edgeValue(sm, box, a1, x.e[1].w), edgeValue(sm, box, a2, x.e[2].w)));
+    return !(lowest < 0.0f) && !(x.t > farT * edgeValue(sm, box, a3, x.e[3].w));
+}
+// the larger depth, NaN if one is (a depth that is not a number rules nothing out)
+__device__ __forceinline__ float farther(float a, float b) {
+    float r;
+    asm("max.NaN.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float warpMin(float v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(kFull, v, o));
+    return v;
+}
+__device__ __forceinline__ float warpMax(float v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
+    return v;
 }
 
 // One tile: intersect, G-buffer grouping, shading and resolve of its 128 samples. The tile's
@@ -621,16 +728,41 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         dv = xformDir(M, f3(b1.z, b1.w, b2.x));
     };
     float dirLen;
-    V2 nc, ndu, ndv; // -c, -du, -dv in both lanes, for the two-triangle setup
+    F3 ncs; // -c
     {
         F3 c, du, dv;
         beamDirs(c, du, dv);
         // Upper bound on |denom| / |e0 x e1| over this sample's subsamples: denom = -dir . n with
         // dir = c + ax du + ay dv and |ax|,|ay| <= 1, so |denom| <= (|c| + |du| + |dv|) |n|.
         dirLen = (sqrtf(dot3(c, c)) + sqrtf(dot3(du, du)) + sqrtf(dot3(dv, dv))) * 1.0001f;
-        nc = V2{pk(-c.x, -c.x), pk(-c.y, -c.y), pk(-c.z, -c.z)};
-        ndu = V2{pk(-du.x, -du.x), pk(-du.y, -du.y), pk(-du.z, -du.z)};
-        ndv = V2{pk(-dv.x, -dv.x), pk(-dv.y, -dv.y), pk(-dv.z, -dv.z)};
+        // footprint radius: the larger singular value of (du dv)
+        const float uu = dot3(du, du), vv = dot3(dv, dv), uv = dot3(du, dv), hd = 0.5f * (uu - vv);
+        const float radius = sqrtf(0.5f * (uu + vv) + sqrtf(hd * hd + uv * uv)) * 1.00002f;
+        // (a beam that is not finite has to pass nothing by: its NaN or infinity must survive the maxima)
+        const float finite = (norm1(c) + norm1(du)) + norm1(dv);
+        const uint32_t r = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? radius : INFINITY));
+        const uint32_t d = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? dirLen : INFINITY));
+        if (tid == 0) {
+            const F3 U = normalize3(du), A = normalize3(dv - U * dot3(U, dv)), W = cross3(U, A);
+            sm.axis[0][0] = U.x; sm.axis[0][1] = U.y; sm.axis[0][2] = U.z;
+            sm.axis[1][0] = A.x; sm.axis[1][1] = A.y; sm.axis[1][2] = A.z;
+            sm.axis[2][0] = W.x; sm.axis[2][1] = W.y; sm.axis[2][2] = W.z;
+        }
+        if (lane == 0) {
+            sm.warpMax[0][warp] = __uint_as_float(r);
+            sm.warpMax[1][warp] = __uint_as_float(d);
+            sm.warpT[warp] = FLT_MAX;
+        }
+        ncs = -c;
+        sm.dir[0][tid] = -du.x; sm.dir[1][tid] = -du.y; sm.dir[2][tid] = -du.z;
+        sm.dir[3][tid] = -dv.x; sm.dir[4][tid] = -dv.y; sm.dir[5][tid] = -dv.z;
+        __syncthreads();
+        // the warp's beams in a box along the axes
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float p = -dot3(c, f3(sm.axis[k][0], sm.axis[k][1], sm.axis[k][2])), lo = warpMin(p), hi = warpMax(p);
+            if (lane == 0) sm.box[k][warp] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * __uint_as_float(d), lo, hi);
+        }
     }
     float tmax[N];
     uint32_t hit[N];
@@ -640,160 +772,209 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         hit[i] = ~0u;
     }
     __syncthreads();
+    const float maxRadius = fmaxf(fmaxf(sm.warpMax[0][0], sm.warpMax[0][1]), fmaxf(sm.warpMax[0][2], sm.warpMax[0][3]));
+    const float maxLen = fmaxf(fmaxf(sm.warpMax[1][0], sm.warpMax[1][1]), fmaxf(sm.warpMax[1][2], sm.warpMax[1][3]));
+    if (tid < 3) {
+        const float lo = fminf(fminf(sm.box[tid][0].z, sm.box[tid][1].z), fminf(sm.box[tid][2].z, sm.box[tid][3].z));
+        const float hi = fmaxf(fmaxf(sm.box[tid][0].w, sm.box[tid][1].w), fmaxf(sm.box[tid][2].w, sm.box[tid][3].w));
+        sm.box[tid][4] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * maxLen, lo, hi);
+    }
+    __syncthreads();
     SHADE_MARK(kScSetup, L.first);
 
-    // The list is consumed chunk by chunk. Entry tid of a chunk is staged into shared memory by
-    // cp.async (the 48-byte triangle record that its index names) while the CTA is still testing
-    // the previous chunk, so the gathers overlap the subsample tests.
+    // Entry tid of a chunk is copied into shared memory by cp.async (the 48-byte triangle record that its
+    // index names) while the CTA is still testing the batch before.
     const float4* __restrict__ trisG = viewPtr(V.tris);
-    auto stage = [&](uint32_t ix) {
-        const float4* src = trisG + 3 * size_t(ix);
-        cpAsync16(&sm.stage[3 * tid + 0], src + 0);
-        cpAsync16(&sm.stage[3 * tid + 1], src + 1);
-        cpAsync16(&sm.stage[3 * tid + 2], src + 2);
-    };
-    uint32_t chunk = L.first;
-    uint32_t remaining = L.count;
-    uint32_t survivors = 0, tested = 0;
-    uint32_t idx = 0;
-    if (chunk < fr.poolChunks && tid < (remaining < kChunk ? remaining : kChunk)) {
-        idx = __ldcg(fr.pool + size_t(chunk) * kChunk + tid);
-        stage(idx);
-    }
-    cpAsyncCommit();
-    while (remaining > 0 && chunk < fr.poolChunks) {
-        const uint32_t n = remaining < kChunk ? remaining : kChunk;
-        const uint32_t nextChunk = __ldcg(fr.chunkNext + chunk);
-        bool keep = false;
-        float t = 0.0f, nlen = 0.0f;
-        F3 e0 = f3(0, 0, 0), e1 = f3(0, 0, 0), v0r = f3(0, 0, 0), nrm = f3(0, 0, 0);
-        cpAsyncWaitAll();
-        if (tid < n) {
-            const float4 ra = sm.stage[3 * tid + 0], rb = sm.stage[3 * tid + 1], rc = sm.stage[3 * tid + 2];
-            const TriGeom tri{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
-            // FrustumPlanes::test
-            bool in = true;
+    uint32_t chunk = L.first, remaining = L.count; // the chunk to copy next and its entries, with all after them
+    uint32_t ready[kBatchChunks], idx[kBatchChunks]; // the copied chunks' entries, this thread's entry of each
+    auto copyBatch = [&] {
 #pragma unroll
-            for (int p = 0; p < 4; p++) {
-                const F3 dir = f3(sm.pl[p][0], sm.pl[p][1], sm.pl[p][2]);
-                const float dist = sm.pl[p][3];
-                const float d0 = dot3(dir, tri.v0);
-                const float d1 = d0 + dot3(dir, tri.e0);
-                const float d2 = d0 + dot3(dir, tri.e1);
-                if (d0 > dist && d1 > dist && d2 > dist) in = false;
+        for (uint32_t b = 0; b < kBatchChunks; b++) {
+            ready[b] = chunk < fr.poolChunks ? (remaining < kChunk ? remaining : kChunk) : 0u;
+            idx[b] = 0;
+            if (tid < ready[b]) {
+                idx[b] = __ldcg(fr.pool + size_t(chunk) * kChunk + tid);
+                const float4* src = trisG + 3 * size_t(idx[b]);
+                for (uint32_t k = 0; k < 3; k++) cpAsync16(&sm.tri[b * kChunk + tid][k], src + k);
             }
-            if (in) {
-                // IntersectTriangleTile<false>::setup
-                const F3 normal = cross3(tri.e0, tri.e1);
-                v0r = camPos - tri.v0;
-                t = dot3(v0r, normal);
-                if (!(t < 0.0f)) {
-                    // TestTriangleFrustaUVW != intersect_all_out
-                    if (!uvwAllOut(sm.ro, sm.rd, tri)) {
-                        keep = true;
-                        e0 = tri.e0;
-                        e1 = tri.e1;
-                        nrm = normal;
-                        nlen = sqrtf(dot3(normal, normal));
+            if (ready[b]) {
+                remaining -= ready[b];
+                chunk = remaining ? __ldcg(fr.chunkNext + chunk) : kNoChunk;
+            }
+        }
+        cpAsyncCommit();
+    };
+    // Triangles that wait to be tested by this lane (kNone: none): when a lane gets a third, or the list
+    // ends, every lane tests those it has, in list order - the first in lane 0 and the second in lane 1
+    // of every packed operation (pairTest). A lone one is tested as the pair (j, j): a second test of the
+    // same triangle on the same subsample changes nothing (it either fails or writes the same depth and
+    // index again).
+    constexpr uint32_t kNone = ~0u;
+    uint32_t wait0 = kNone, wait1 = kNone;
+    float laneT = FLT_MAX; // the largest depth of the lane's subsamples
+    uint32_t survivors = 0, tested = 0, lanesTested = 0;
+    copyBatch();
+    for (bool more = true; more;) {
+        // Which entries of the batch can meet the tile: the triangle's planes against the tile's box of beams
+        uint32_t kept = 0;
+        const float tileT = farther(farther(sm.warpT[0], sm.warpT[1]), farther(sm.warpT[2], sm.warpT[3]));
+        cpAsyncWaitAll();
+#pragma unroll
+        for (uint32_t b = 0; b < kBatchChunks; b++) {
+            bool keep = false;
+            const uint32_t slot = b * kChunk + tid;
+            if (tid < ready[b]) {
+                const float4 ra = sm.tri[slot][0], rb = sm.tri[slot][1], rc = sm.tri[slot][2];
+                const TriGeom tri{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
+                const TriPlanes x = trianglePlanes(tri, camPos, maxRadius, maxLen);
+                if (!(x.t < 0.0f)) // IntersectTriangleTile<false>::setup
+                    keep = planesMeet(sm, 4, edgeAlong(sm, x.e[0]), edgeAlong(sm, x.e[1]), edgeAlong(sm, x.e[2]),
+                                      edgeAlong(sm, x.e[3]), x, tileT);
+            }
+            const uint32_t bal = __ballot_sync(kFull, keep);
+            if (lane == 0) sm.warpCount[b][warp] = __popc(bal);
+            kept |= (keep ? 1u : 0u) << b;
+            if (keep) sm.tri[slot][2].y = __uint_as_float(idx[b]); // (a triangle row's last three words are unused)
+        }
+        __syncthreads();
+        uint32_t have = 0;
+#pragma unroll
+        for (uint32_t b = 0; b < kBatchChunks; b++) {
+            const uint32_t bal = __ballot_sync(kFull, (kept >> b) & 1u);
+            uint32_t off = have + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+            for (uint32_t w = 0; w < 4; w++) {
+                const uint32_t cw = sm.warpCount[b][w];
+                off += (w < warp) ? cw : 0u;
+                have += cw;
+            }
+            if ((kept >> b) & 1u) sm.cand[off] = uint16_t(b * kChunk + tid);
+        }
+        __syncthreads();
+        SHADE_MARK(kScCull, have);
+        for (uint32_t first = 0; first == 0 || first < have; first += kChunk) {
+            // The tile's own tests on those, one per thread, and which warps need them. The depth bounds are
+            // the last round's; depths only fall, so they skip no triangle that could hit.
+            const uint32_t groups = first < have ? (min(have - first, kChunk) + 31u) / 32u : 0u;
+            if (warp < groups) {
+                const uint32_t js = first + tid;
+                uint32_t warps = 0;
+                if (js < have) {
+                    const uint32_t slot = sm.cand[js];
+                    const float4 ra = sm.tri[slot][0], rb = sm.tri[slot][1], rc = sm.tri[slot][2];
+                    const TriGeom tj{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
+                    const TriPlanes x = trianglePlanes(tj, camPos, maxRadius, maxLen);
+                    const F3 a0 = edgeAlong(sm, x.e[0]), a1 = edgeAlong(sm, x.e[1]), a2 = edgeAlong(sm, x.e[2]), a3 = edgeAlong(sm, x.e[3]);
+#pragma unroll
+                    for (uint32_t w = 0; w < 4; w++)
+                        if (planesMeet(sm, w, a0, a1, a2, a3, x, sm.warpT[w])) warps |= 1u << w;
+                    // FrustumPlanes::test, TestTriangleFrustaUVW != intersect_all_out
+                    if (warps && !(inFrustum(sm.pl, tj) && !uvwAllOut(sm.ro, sm.rd, tj))) warps = 0;
+                    if (warps) {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) sm.edge[e][tid] = x.e[e];
+                        sm.t[tid] = x.t;
+                        sm.idx[tid] = __float_as_uint(rc.y);
                     }
                 }
-            }
-        }
-        // the next chunk's index of this entry (its chunk link has arrived by now)
-        const uint32_t rest = remaining - n;
-        const bool more = rest > 0 && nextChunk < fr.poolChunks;
-        uint32_t idxNext = 0;
-        if (more && tid < (rest < kChunk ? rest : kChunk)) idxNext = __ldcg(fr.pool + size_t(nextChunk) * kChunk + tid);
-        const uint32_t bal = __ballot_sync(kFull, keep);
-        if (lane == 0) sm.warpCount[warp] = __popc(bal);
-        __syncthreads();
-        uint32_t off = __popc(bal & ((1u << lane) - 1u));
-        uint32_t total = 0;
+                survivors += __popc(__ballot_sync(kFull, warps != 0));
 #pragma unroll
-        for (uint32_t w = 0; w < 4; w++) {
-            const uint32_t cw = sm.warpCount[w];
-            off += (w < warp) ? cw : 0u;
-            total += cw;
-        }
-        if (keep) {
-            sm.g[0][off] = e0.x; sm.g[1][off] = e0.y; sm.g[2][off] = e0.z;
-            sm.g[3][off] = e1.x; sm.g[4][off] = e1.y; sm.g[5][off] = e1.z;
-            sm.g[6][off] = v0r.x; sm.g[7][off] = v0r.y; sm.g[8][off] = v0r.z;
-            sm.g[9][off] = nrm.x; sm.g[10][off] = nrm.y; sm.g[11][off] = nrm.z;
-            sm.t[off] = t;
-            sm.nlen[off] = nlen;
-            sm.idx[off] = idx;
-        }
-        __syncthreads();
-        SHADE_MARK(kScCull, total);
-        // stage the next chunk (this thread's entry of this chunk was read above)
-        if (more && tid < (rest < kChunk ? rest : kChunk)) stage(idxNext);
-        cpAsyncCommit();
-        // Depth skip. The test rejects a subsample when depth * denom < t (FMA mode, exactly;
-        // STRICT mode with the product rounded, covered by the 1e-4 margin in dirLen). With
-        // denom <= dirLen * |n| and depth <= laneT, t > laneT * dirLen * |n| rejects every
-        // subsample of the lane; a triangle is skipped only when that holds for all 32 lanes, so
-        // the hits are exactly those of the full loop. Misses keep laneT at FLT_MAX (no skip).
-        // For |n| >= 0 the rounded product is monotone in the bound, so "for all lanes" is the
-        // test against the warp's largest bound, and lane l evaluates it for survivor g + l: one
-        // ballot decides 32 survivors. The bound is taken at the start of each group of 32; depths
-        // only fall, so a bound taken earlier is larger and skips no triangle that could hit.
-        //
-        // The triangles that are not skipped are tested two at a time, in list order: j in lane 0
-        // and k in lane 1 of every packed operation (pairTest). An odd one left at the end of the
-        // chunk is tested as the pair (j, j): a second test of the same triangle on the same
-        // subsample changes nothing (it either fails or writes the same depth and index again).
-        survivors += total;
-        uint32_t pend = ~0u; // a triangle waiting for its pair partner
-        auto testPair = [&](uint32_t j, uint32_t k) {
-            const V2 e0 = {pk(sm.g[0][j], sm.g[0][k]), pk(sm.g[1][j], sm.g[1][k]), pk(sm.g[2][j], sm.g[2][k])};
-            const V2 e1 = {pk(sm.g[3][j], sm.g[3][k]), pk(sm.g[4][j], sm.g[4][k]), pk(sm.g[5][j], sm.g[5][k])};
-            const V2 vr = {pk(sm.g[6][j], sm.g[6][k]), pk(sm.g[7][j], sm.g[7][k]), pk(sm.g[8][j], sm.g[8][k])};
-            const V2 nn = {pk(sm.g[9][j], sm.g[9][k]), pk(sm.g[10][j], sm.g[10][k]), pk(sm.g[11][j], sm.g[11][k])};
-            const float tj = sm.t[j], tk = sm.t[k];
-            const uint32_t ij = sm.idx[j], ik = sm.idx[k];
-            const TriPair tp = pairSetup(nn, e0, e1, vr, nc, ndu, ndv);
-            const P2 tt = FMA ? pk(-tj, -tk) : pk(tj, tk);
-#pragma unroll
-            for (uint32_t i = 0; i < N; i++) {
-                const P2 ax = *reinterpret_cast<const P2*>(&cMsaaXX[rate][i]);
-                const P2 ay = *reinterpret_cast<const P2*>(&cMsaaYY[rate][i]);
-                pairTest<FMA>(tp, tt, tj, tk, ij, ik, ax, ay, tmax[i], hit[i]);
-            }
-        };
-        for (uint32_t g0 = 0; g0 < total; g0 += 32) {
-            float laneT = 0.0f;
-#pragma unroll
-            for (uint32_t i = 0; i < N; i++) laneT = fmaxf(laneT, tmax[i]);
-            const float bound = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(laneT * dirLen)));
-            const uint32_t js = g0 + lane;
-            const bool skip = js < total && sm.t[js] > bound * sm.nlen[js];
-            uint32_t live = __ballot_sync(kFull, js < total && !skip);
-            tested += __popc(live);
-            while (live) {
-                const uint32_t j = g0 + uint32_t(__ffs(live) - 1);
-                live &= live - 1u;
-                if (pend == ~0u) {
-                    pend = j;
-                } else {
-                    testPair(pend, j);
-                    pend = ~0u;
+                for (uint32_t w = 0; w < 4; w++) {
+                    const uint32_t b = __ballot_sync(kFull, (warps >> w) & 1u);
+                    if (lane == w) sm.need[warp][w] = b;
                 }
             }
+            const bool last = first + kChunk >= have; // (of the batch)
+            __syncthreads();
+            if (last) {
+                copyBatch();
+                more = ready[0] != 0;
+            }
+            auto mayHit = [&](uint32_t slot) {
+                const float lowest = fminf(edgeValue(ncs, sm.edge[0][slot]),
+                                           fminf(edgeValue(ncs, sm.edge[1][slot]), edgeValue(ncs, sm.edge[2][slot])));
+                return !(lowest < 0.0f) && !(sm.t[slot] > laneT * edgeValue(ncs, sm.edge[3][slot]));
+            };
+            uint32_t g = 0, mine = 0; // mine: the group's triangles that the lane still has to take
+            for (;;) {
+                if (!__any_sync(kFull, mine != 0)) {
+                    if (g == groups) {
+                        if (more || !last) break;
+                    } else {
+                        // every lane decides which of its warp's triangles its own sample needs (two at a time;
+                        // an odd one twice)
+                        for (uint32_t live = sm.need[g][warp]; live;) {
+                            const uint32_t b0 = uint32_t(__ffs(live) - 1);
+                            live &= live - 1u;
+                            const uint32_t b1 = live ? uint32_t(__ffs(live) - 1) : b0;
+                            live &= live - 1u;
+                            const bool p0 = mayHit(g * 32u + b0), p1 = mayHit(g * 32u + b1);
+                            mine |= (p0 ? 1u << b0 : 0u) | (p1 ? 1u << b1 : 0u);
+                        }
+                        tested += __popc(__reduce_or_sync(kFull, mine));
+                        g++;
+                    }
+                }
+                // take up to two
+                for (int k = 0; k < 2; k++)
+                    if (mine && wait1 == kNone) {
+                        const uint32_t tri = sm.idx[(g - 1u) * 32u + uint32_t(__ffs(mine) - 1)];
+                        mine &= mine - 1u;
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(trisG + 3 * size_t(tri)));
+                        if (wait0 == kNone) wait0 = tri;
+                        else wait1 = tri;
+                    }
+                const bool end = g == groups && !more && last && !__any_sync(kFull, mine != 0);
+                if (__any_sync(kFull, end ? wait0 != kNone : mine != 0)) {
+                    if (wait0 != kNone) {
+                        const uint32_t ij = wait0, ik = wait1 == kNone ? wait0 : wait1;
+                        lanesTested += wait1 == kNone ? 1u : 2u;
+                        const float4* rj = trisG + 3 * size_t(ij);
+                        const float4* rk = trisG + 3 * size_t(ik);
+                        const float4 j0 = __ldg(rj), j1 = __ldg(rj + 1), k0 = __ldg(rk), k1 = __ldg(rk + 1);
+                        const float j2 = __ldg(&rj[2].x), k2 = __ldg(&rk[2].x);
+                        const V2 e0 = {pk(j0.w, k0.w), pk(j1.x, k1.x), pk(j1.y, k1.y)};
+                        const V2 e1 = {pk(j1.z, k1.z), pk(j1.w, k1.w), pk(j2, k2)};
+                        const V2 vr = {pk(camPos.x - j0.x, camPos.x - k0.x), pk(camPos.y - j0.y, camPos.y - k0.y),
+                                       pk(camPos.z - j0.z, camPos.z - k0.z)};
+                        const V2 nn = cross2(e0, e1);
+                        const P2 t2 = dot2(vr, nn);
+                        float tj, tk;
+                        upk(t2, tj, tk);
+                        const F3 du = f3(sm.dir[0][tid], sm.dir[1][tid], sm.dir[2][tid]), dv = f3(sm.dir[3][tid], sm.dir[4][tid], sm.dir[5][tid]);
+                        const TriPair tp = pairSetup(nn, e0, e1, vr, V2{pk(ncs.x, ncs.x), pk(ncs.y, ncs.y), pk(ncs.z, ncs.z)},
+                                                     V2{pk(du.x, du.x), pk(du.y, du.y), pk(du.z, du.z)},
+                                                     V2{pk(dv.x, dv.x), pk(dv.y, dv.y), pk(dv.z, dv.z)});
+                        const P2 tt = FMA ? neg2(t2) : t2;
+#pragma unroll
+                        for (uint32_t i = 0; i < N; i++) {
+                            const P2 ax = *reinterpret_cast<const P2*>(&cMsaaXX[rate][i]);
+                            const P2 ay = *reinterpret_cast<const P2*>(&cMsaaYY[rate][i]);
+                            pairTest<FMA>(tp, tt, tj, tk, ij, ik, ax, ay, tmax[i], hit[i]);
+                        }
+                        laneT = 0.0f;
+#pragma unroll
+                        for (uint32_t i = 0; i < N; i++) laneT = farther(laneT, tmax[i]);
+                        wait0 = wait1 = kNone;
+                    }
+                    __syncwarp();
+                }
+                if (end) break;
+            }
+            const uint32_t far = __reduce_max_sync(kFull, __float_as_uint(laneT));
+            if (lane == 0) sm.warpT[warp] = __uint_as_float(far);
+            __syncthreads();
         }
-        if (pend != ~0u) testPair(pend, pend);
-        __syncthreads();
-        remaining -= n;
-        chunk = nextChunk;
-        idx = idxNext;
         SHADE_MARK(kScTest, remaining);
 #ifdef HVVR_VISIT_CLOCKS
-        ++scChunks;
+        scChunks += kBatchChunks;
 #endif
     }
 
-    if (tid == 0 && survivors) atomicAdd(&fr.counters[kSurvivorWord], survivors);
+    if (lane == 0 && survivors) atomicAdd(&fr.counters[kSurvivorWord], survivors);
     if (lane == 0 && tested) atomicAdd(&fr.counters[kTestedWord], tested);
+    lanesTested = __reduce_add_sync(kFull, lanesTested);
+    if (lane == 0 && lanesTested) atomicAdd(&fr.counters[kSampleTestedWord], lanesTested);
     F3 c, du, dv;
     beamDirs(c, du, dv);
     if (uint32_t* hitOut = viewPtr(V.hitIds)) {

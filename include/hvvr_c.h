@@ -493,10 +493,11 @@ int hvvr_batch_read_stats(const hvvr_batch* batch, uint64_t* out4);
 /* The last frame's counters, out[0..count): [0] triangle-list pool entries used (whole chunks),
  * [1] tiles culled again with the 4096-entry stack, [2] status bits, [3] views, [4] list entries
  * that passed the intersect's per-tile tests (frustum planes, ray-origin side, corner-ray
- * barycentrics), [5] (warp of 32 samples, passing entry) pairs whose subsample tests ran (the
- * intersect skips a pair when a depth bound proves that no subsample of the warp can hit the
- * triangle, so [5] x 32 samples x msaa is the number of subsample tests executed, at most
- * [4] x 4 warps); later indices read 0. */
+ * barycentrics, and the bounds on what the tile's samples can still hit), [5] (warp of 32 samples,
+ * passing entry) pairs of which some sample's subsample tests ran, [6] (sample, passing entry) pairs
+ * whose subsample tests ran (the intersect passes a pair by when its footprint and depth bounds prove
+ * that no subsample can hit the triangle, so [6] x msaa is the number of subsample tests executed);
+ * later indices read 0. */
 int hvvr_batch_read_counters(const hvvr_batch* batch, uint64_t* out, uint32_t count);
 int hvvr_raycaster_read_counters(const hvvr_raycaster* rc, uint64_t* out, uint32_t count);
 
