@@ -164,7 +164,10 @@ Instance* makeInstance(hvvr_server* s, uint32_t t) {
     inst->tmpl = t;
     inst->width = tp.width;
     inst->height = tp.height;
-    if (inst->image.alloc(size_t(tp.width) * tp.height) != HVVR_OK) {
+    // pixels that no sample maps to are never written: they are black, not what the memory held
+    if (inst->image.alloc(size_t(tp.width) * tp.height) != HVVR_OK ||
+        cudaMemsetAsync(inst->image.p, 0, size_t(tp.width) * tp.height * 4, cam->rc->stream) != cudaSuccess ||
+        cudaStreamSynchronize(cam->rc->stream) != cudaSuccess) {
         hvvr_camera_destroy(cam->rc, cam);
         return nullptr;
     }
