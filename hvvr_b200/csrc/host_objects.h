@@ -9,6 +9,7 @@
 
 #include <atomic>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -73,6 +74,15 @@ struct DevBuf {
         return HVVR_OK;
     }
 };
+
+// A raycaster's scratch for device sample setups: about 60 bytes a sample, kept between builds up to
+// kSetupScratchKept (4 million samples) and freed with the raycaster. Builds of one raycaster's cameras
+// take turns, each until its work on the device is done.
+struct SetupScratch {
+    std::mutex mutex;
+    DevBuf<uint8_t> buf;
+};
+constexpr size_t kSetupScratchKept = size_t(256) << 20;
 
 // A 2D CUDA array with a texture object (reads) and a surface object (writes), made as the
 // reference's createEmptyTexture makes one (libraries/hvvr/raycaster/texture.cu:283-321):
@@ -248,6 +258,7 @@ struct hvvr_raycaster {
     DevBuf<Mat4> modelToWorld;
     std::vector<Node> hostNodes;
     uint32_t refitStatus = 0;
+    SetupScratch setupScratch;
     std::unique_ptr<hvvr_batch> own;      // renders this raycaster's cameras
     std::unique_ptr<PolarSetup> polar;    // foveated polar mode: the sample set of spec's pattern
     std::vector<hvvr_batch*> batches;     // user batches that include this raycaster

@@ -258,10 +258,12 @@ int setupCamera(hvvr_camera* cam, cudaStream_t st) {
     // the sample hierarchy: on the device unless the spec asks for the host, the spherical
     // mapping is on (its sin/cos follow the host's libm), or two samples share a position
     bool host = cam->rc->spec.sample_setup == HVVR_SETUP_HOST || cam->fovX > 0.0f;
+    // a frame of the camera may still be reading the buffers that the new setup is written to
+    if (cam->lastBatch && cam->lastBatch->ev[5]) CUDA_TRY(cudaStreamWaitEvent(st, cam->lastBatch->ev[5], 0));
     if (!host) {
         DeviceSampleSetup ds{&cam->tileRays, &cam->blockRays, &cam->beams, &cam->remap};
         TRY(buildSampleSetupDevice(cam->samples.data(), uint32_t(cam->samples.size()), cam->split, cam->viewport,
-                                   cam->lens, w, h, ds, st, host));
+                                   cam->lens, w, h, cam->rc->setupScratch, ds, st, host));
         if (!host) {
             cam->setup = SampleSetup{};
             cam->setup.blocks = ds.blocks;
@@ -293,7 +295,11 @@ int setupCamera(hvvr_camera* cam, cudaStream_t st) {
     TRY(cam->tileCost.alloc(ss.tiles));
     CUDA_TRY(cudaMemsetAsync(cam->tileCost.p, 0, size_t(ss.tiles) * 4, st));
     const bool cpuTarget = cam->target.memory_type == HVVR_MEMORY_CPU;
-    if (cpuTarget && w && h) TRY(cam->image.alloc(size_t(w) * h));
+    if (cpuTarget && w && h && cam->image.n != size_t(w) * h) {
+        // pixels that no sample maps to are never written: they are black, not what the memory held
+        TRY(cam->image.alloc(size_t(w) * h));
+        CUDA_TRY(cudaMemsetAsync(cam->image.p, 0, size_t(w) * h * 4, st));
+    }
     CameraDev& d = cam->dev;
     d.blocks = ss.blocks;
     d.tiles = ss.tiles;

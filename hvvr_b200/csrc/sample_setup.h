@@ -21,12 +21,14 @@ struct DeviceSampleSetup {
     uint32_t blocks = 0, tiles = 0, padded = 0, valid = 0;
 };
 
+struct SetupScratch; // host_objects.h
+
 // SampleData for the perspective mapping, on the device: clusters the samples, and writes the
 // tile and block frusta (camera space), the beams and the image -> sample remap. needsHost is set
-// (and nothing written) when two samples share a position or a position is NaN: the reference's
+// (and what was written is to be replaced) when two samples share a position or a position is NaN: the reference's
 // std::sort then decides their order, and the caller builds on the host.
 int buildSampleSetupDevice(const hvvr_sample* samples, uint32_t count, uint32_t split, const hvvr_float_rect& vp,
-                           const hvvr_thin_lens& lens, uint32_t width, uint32_t height, DeviceSampleSetup& out,
-                           cudaStream_t st, bool& needsHost);
+                           const hvvr_thin_lens& lens, uint32_t width, uint32_t height, SetupScratch& scratch,
+                           DeviceSampleSetup& out, cudaStream_t st, bool& needsHost);
 
 } // namespace hvb
