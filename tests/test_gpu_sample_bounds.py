@@ -64,3 +64,28 @@ def test_bounds_change_no_hit(oracle, name, scale, w, h, msaa, eye, target, fp_m
         assert d.max() <= 1
     assert (ids != 0xFFFFFFFF).any()
     rc.close()
+
+
+@pytest.mark.parametrize("fp_mode", [hv.HVVR_FP_FMA, hv.HVVR_FP_STRICT])
+@pytest.mark.parametrize("name,scale,w,h,msaa,lens,eye,target", [
+    ("c1", 1.0, 64, 48, 4, (0.002, 9.0), (0.0, 2.0, 10.0), (0.0, 0.0, 0.0)),   # hardly any blur
+    ("c1", 1.0, 96, 72, 8, (0.5, 3.0), (0.0, 2.0, 10.0), (0.0, 0.0, 0.0)),     # focused before the scene
+    ("small", 1.0, 97, 61, 1, (0.3, 40.0), (3.0, 1.5, 8.0), (0.0, 0.0, 0.0)),  # focused behind it
+    ("room", 1.0, 128, 96, 16, (0.1, 8.0), (0.0, 2.0, 9.0), (0.0, 0.0, 0.0)),
+    ("small", 1e4, 96, 64, 8, (400.0, 9e4), (0.0, 2.0, 10.0), (0.0, 0.0, 0.0)),
+    ("small", 1e-4, 96, 64, 2, (4e-6, 9e-4), (0.0, 2.0, 10.0), (0.0, 0.0, 0.0)),
+    ("doubled", 1.0, 80, 60, 4, (0.05, 7.0), (1.0, 0.6, 3.0), (0.0, -0.5, 0.0)),
+])
+def test_lens_bounds_change_no_hit(oracle, name, scale, w, h, msaa, lens, eye, target, fp_mode):
+    sc = _scaled(_scene(name), scale)
+    xf = scenes.camera_transform(tuple(scale * x for x in eye), tuple(scale * x for x in target))
+    smp = scenes.barrel_samples(w, h)
+    rc, cam = render_gpu(sc, smp, w, h, msaa, xf, fp_mode, lens=lens)
+    ids, depth = cam.hits()
+    fo = render_oracle(oracle, sc, smp, w, h, msaa, xf, fp_mode, lens=lens)
+    assert np.array_equal(ids, fo.hit_ids)
+    assert np.array_equal(depth.view(np.uint32), fo.depth.view(np.uint32))
+    d = np.abs(cam.sample_colors().view(np.uint8).astype(int) - fo.colors.view(np.uint8).astype(int))
+    assert d.max() <= 1
+    assert (ids != 0xFFFFFFFF).any()
+    rc.close()
