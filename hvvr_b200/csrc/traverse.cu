@@ -1293,14 +1293,6 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
         sync();
         return visits;
     }
-    // the list's chunks, consecutive in the pool
-    const uint32_t chunks = (total + kChunk - 1) / kChunk;
-    uint32_t chunk0 = 0;
-    if (tid == 0) {
-        chunk0 = atomicAdd(&a.counters[0], chunks);
-        if (W > 1) h.first = chunk0;
-    }
-    __syncwarp();
     // depth-first offsets inside the components: subtree sizes upwards, offsets downwards
     for (uint32_t g = gens; g-- > 0;) {
         for (uint32_t i = h.gen[g] + tid; i < h.gen[g + 1]; i += G) {
@@ -1359,11 +1351,19 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
     sync();
     if constexpr (W > 1) sorted = h.sorted;
     if (sorted > S::kSorted) {
-        // (its chunks stay allocated and unused)
         overflow = true;
         sync();
         return visits;
     }
+    // the list's chunks, consecutive in the pool: taken once nothing can send the tile to another cull any
+    // more, so that a pool that holds the lists is always enough
+    const uint32_t chunks = (total + kChunk - 1) / kChunk;
+    uint32_t chunk0 = 0;
+    if (tid == 0) {
+        chunk0 = atomicAdd(&a.counters[0], chunks);
+        if (W > 1) h.first = chunk0;
+    }
+    __syncwarp();
     groupSort<W>(s.sortKey, sorted, wid, sync);
     // runs of equal keys in their exact order
     uint16_t* ordered = s.first;
@@ -1612,7 +1612,8 @@ constexpr uint32_t kOrderPerThread = (kOrderBuckets + 1023) / 1024;
 __host__ __device__ constexpr uint32_t costBucket(uint32_t c, uint32_t log2) { return kCostBuckets - 1 - (log2 * 4 + (((c + 1) << (31 - log2)) >> 29 & 3u)); }
 // A tile of at least kBigCost visits is culled by a whole CTA and one of at least kHugeCost by a CTA
 // with an SM's shared memory: bucket bounds that leave a warp's store (kWarpNodes) a third and a
-// CTA's (kCtaNodes) an eighth of headroom for a view that moves between frames (a huge tile holds a
+// CTA's (kCtaNodes) an eighth of headroom for a view that moves between frames (a tile of which more than
+// half of the store's nodes are list-bearing components outgrows the store earlier; a huge tile holds a
 // whole SM: starting them at 1,536 visits took 6.0 ms instead of 2.8 for the cull of a foveated
 // frame with a thousand of them).
 constexpr uint32_t kBigCost = 191, kHugeCost = 1791;
