@@ -605,6 +605,23 @@ __device__ __forceinline__ F3 cross3fma(F3 a, F3 b) {
     return f3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
 }
 __device__ __forceinline__ float edgeValue(F3 nc, float4 e) { return fmaf(nc.x, e.x, fmaf(nc.y, e.y, fmaf(nc.z, e.z, e.w))); }
+// Orthonormal axes about along du and dv, to a few half-ulps whatever du and dv are: the boxes' 1e-6 of the
+// beam length is all that their error may cost. One step of dv - U (U . dv) leaves a share of U that grows as
+// du and dv near each other (a viewport scaled very unequally under rotated ellipses), hence the second. A
+// direction lost to rounding, to squares below the normal range, or because it is zero, is replaced.
+__device__ __forceinline__ void boxAxes(F3 du, F3 dv, F3& U, F3& A, F3& W) {
+    U = normalize3(du);
+    if (!(fabsf(dot3(U, U) - 1.0f) < 1e-5f)) U = f3(1.0f, 0.0f, 0.0f);
+    A = normalize3(dv - U * dot3(U, dv));
+    A = A - U * dot3(U, A);
+    if (!(dot3(A, A) > 0.5f && dot3(A, A) <= 2.0f)) { // the coordinate axis farthest from U, without its share of U
+        const float x = fabsf(U.x), y = fabsf(U.y), z = fabsf(U.z);
+        A = x <= y && x <= z ? f3(1.0f, 0.0f, 0.0f) : (y <= z ? f3(0.0f, 1.0f, 0.0f) : f3(0.0f, 0.0f, 1.0f));
+        A = A - U * dot3(U, A);
+    }
+    A = normalize3(A);
+    W = cross3(U, A);
+}
 // a plane's components along the tile's axes, and its value over a box of beams (its largest)
 __device__ __forceinline__ F3 edgeAlong(const ShadeSmem& sm, float4 e) {
     const F3 g = f3(e.x, e.y, e.z);
@@ -746,7 +763,8 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         const uint32_t r = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? radius : INFINITY));
         const uint32_t d = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? dirLen : INFINITY));
         if (tid == 0) {
-            const F3 U = normalize3(du), A = normalize3(dv - U * dot3(U, dv)), W = cross3(U, A);
+            F3 U, A, W;
+            boxAxes(du, dv, U, A, W);
             sm.axis[0][0] = U.x; sm.axis[0][1] = U.y; sm.axis[0][2] = U.z;
             sm.axis[1][0] = A.x; sm.axis[1][1] = A.y; sm.axis[1][2] = A.z;
             sm.axis[2][0] = W.x; sm.axis[2][1] = W.y; sm.axis[2][2] = W.z;
