@@ -253,13 +253,14 @@ int setupFoveatedCamera(hvvr_camera* cam, cudaStream_t st);
 
 int setupCamera(hvvr_camera* cam, cudaStream_t st) {
     if (cam->samples.empty()) return fail(HVVR_ERR_STATE, "camera has no samples");
+    // a frame of the camera may still be reading what the new setup writes (a foveated camera's textures too,
+    // which are made anew once the host has waited for st)
+    if (cam->lastBatch && cam->lastBatch->ev[5]) CUDA_TRY(cudaStreamWaitEvent(st, cam->lastBatch->ev[5], 0));
     if (cam->rc->spec.mode == HVVR_MODE_FOVEATED_POLAR) return setupFoveatedCamera(cam, st);
     const uint32_t w = cam->target.width, h = cam->target.height;
     // the sample hierarchy: on the device unless the spec asks for the host, the spherical
     // mapping is on (its sin/cos follow the host's libm), or two samples share a position
     bool host = cam->rc->spec.sample_setup == HVVR_SETUP_HOST || cam->fovX > 0.0f;
-    // a frame of the camera may still be reading the buffers that the new setup is written to
-    if (cam->lastBatch && cam->lastBatch->ev[5]) CUDA_TRY(cudaStreamWaitEvent(st, cam->lastBatch->ev[5], 0));
     if (!host) {
         DeviceSampleSetup ds{&cam->tileRays, &cam->blockRays, &cam->beams, &cam->remap};
         TRY(buildSampleSetupDevice(cam->samples.data(), uint32_t(cam->samples.size()), cam->split, cam->viewport,
