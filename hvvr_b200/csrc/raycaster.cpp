@@ -296,8 +296,9 @@ int setupCamera(hvvr_camera* cam, cudaStream_t st) {
     TRY(cam->tileCost.alloc(ss.tiles));
     CUDA_TRY(cudaMemsetAsync(cam->tileCost.p, 0, size_t(ss.tiles) * 4, st));
     const bool cpuTarget = cam->target.memory_type == HVVR_MEMORY_CPU;
-    if (cpuTarget && w && h && cam->image.n != size_t(w) * h) {
-        // pixels that no sample maps to are never written: they are black, not what the memory held
+    if (cpuTarget && w && h) {
+        // pixels that no sample maps to are never written: they are black, not what the memory held or the
+        // samples before drew there
         TRY(cam->image.alloc(size_t(w) * h));
         CUDA_TRY(cudaMemsetAsync(cam->image.p, 0, size_t(w) * h * 4, st));
     }

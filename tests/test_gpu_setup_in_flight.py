@@ -64,3 +64,32 @@ def test_setup_waits_for_running_frames(foveated):
     rc.synchronize()
     stream.synchronize()
     rc.close()
+
+
+def test_new_samples_start_from_a_black_image():
+    """Pixels that no sample of the new set maps to are black, not what the set before drew there."""
+    sc = scene("c1")
+    rc = hv.Raycaster()
+    rc.create_model(sc)
+    for light in sc.lights:
+        rc.create_light(light)
+    cam = rc.create_camera(scenes.viewport_for(W, H))
+    cam.set_render_target(W, H)
+    cam.set_camera_to_world(scenes.camera_transform())
+    cam.set_msaa(4)
+    full = scenes.grid_samples(W, H)
+    for shape in ((W, H), (H, W)):  # as many pixels in another shape
+        cam.set_render_target(*shape)
+        cam.set_samples(full)
+        rc.render()
+        rc.synchronize()
+        assert (cam.image != 0).sum() > 0
+        half = full[full["pixel"][:, 0] < 100]
+        cam.set_samples(half)
+        rc.render()
+        rc.synchronize()
+        drawn = np.zeros(cam.image.shape, bool)
+        on = half[(half["pixel"][:, 0] < shape[0]) & (half["pixel"][:, 1] < shape[1])]
+        drawn[on["pixel"][:, 1], on["pixel"][:, 0]] = True
+        assert (cam.image[~drawn] == 0).all() and (cam.image[drawn] != 0).any()
+    rc.close()
