@@ -1113,6 +1113,57 @@ __device__ void groupSort(unsigned long long* v, uint32_t n, uint32_t wid, Sync 
     }
 }
 
+// Components with equal sort keys are ordered by counting what comes before each, a comparison for every pair
+// of a run. Where one root's key exceeds every key below it (the block's axis differs from the tile's, in a
+// scene far from the origin) all of that root's components are one run, so a tile with a run longer than this is
+// merged instead, by the kernel whose CTA has an SM (the other has no registers for it). One root of 1,783 and
+// of 6,657 nodes, 128 tiles: 2,563 and 4,453 us by counting, 497 and 832 us by merging, 577 and 718
+// without ties.
+constexpr uint32_t kLongRun = 256;
+
+// The components of s.sortKey into s.first in their exact order: merge passes over blocks of 1, 2, 4, ... of each
+// run of equal keys, each element finding its place in the other block by bisection.
+template <int W, class S>
+__device__ __noinline__ void mergeRuns(S& s, const uint32_t* rootKey, uint32_t sorted) {
+    uint16_t *from = s.first, *to = s.first + S::kSorted;
+    // the first position whose key is not below k
+    auto bound = [&](uint64_t k) {
+        uint32_t lo = 0, hi = sorted;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if ((s.sortKey[mid] >> 32) < k) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    for (uint32_t e = threadIdx.x; e < sorted; e += 32 * W) from[e] = uint16_t(s.sortKey[e]);
+    __syncthreads();
+    for (uint32_t width = 1; width < sorted; width *= 2) {
+        for (uint32_t e = threadIdx.x; e < sorted; e += 32 * W) {
+            const uint64_t key = s.sortKey[e] >> 32;
+            const uint32_t id = from[e], begin = bound(key), end = bound(key + 1);
+            const uint32_t low = begin + ((e - begin) & ~(2 * width - 1)), mid = min(low + width, end);
+            const bool left = e < mid;
+            uint32_t b = left ? mid : low, t = left ? min(mid + width, end) : mid;
+            const uint32_t other = b;
+            while (b < t) {
+                const uint32_t m = (b + t) / 2;
+                if (compBefore(s, rootKey, from[m], id)) b = m + 1;
+                else t = m;
+            }
+            to[low + (e - (left ? low : mid)) + (b - other)] = uint16_t(id);
+        }
+        __syncthreads();
+        uint16_t* const f = from;
+        from = to;
+        to = f;
+    }
+    if (from != s.first) {
+        for (uint32_t e = threadIdx.x; e < sorted; e += 32 * W) to[e] = from[e];
+        __syncthreads();
+    }
+}
+
 // one tile by W warps (W = 1: the calling warp alone; else the whole CTA); returns the node visits.
 // overflow: the list was not made (see above).
 template <int W, uint32_t N>
@@ -1355,22 +1406,19 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
         sync();
         return visits;
     }
-    // the list's chunks, consecutive in the pool: taken once nothing can send the tile to another cull any
-    // more, so that a pool that holds the lists is always enough
-    const uint32_t chunks = (total + kChunk - 1) / kChunk;
-    uint32_t chunk0 = 0;
-    if (tid == 0) {
-        chunk0 = atomicAdd(&a.counters[0], chunks);
-        if (W > 1) h.first = chunk0;
-    }
-    __syncwarp();
     groupSort<W>(s.sortKey, sorted, wid, sync);
     // runs of equal keys in their exact order
     uint16_t* ordered = s.first;
+    bool longRun = false; // (a warp's are short)
     for (uint32_t e = tid; e < sorted; e += G) {
         const unsigned long long v = s.sortKey[e];
         const uint32_t key = uint32_t(v >> 32), id = uint32_t(v);
         uint32_t pos = e;
+        if (W > 1 && ((e >= kLongRun && uint32_t(s.sortKey[e - kLongRun] >> 32) == key) ||
+                      (e + kLongRun < sorted && uint32_t(s.sortKey[e + kLongRun] >> 32) == key))) {
+            longRun = true;
+            continue;
+        }
         for (uint32_t j = e; j-- > 0;) {
             const unsigned long long o = s.sortKey[j];
             if (uint32_t(o >> 32) != key) break;
@@ -1383,7 +1431,25 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
         }
         ordered[pos] = uint16_t(id);
     }
-    sync();
+    if constexpr (W == 1) {
+        __syncwarp();
+    } else if (__syncthreads_or(longRun)) {
+        if constexpr (W < int(kHugeWarps)) { // (left to the kernel that merges)
+            overflow = true;
+            return visits;
+        } else {
+            mergeRuns<W>(s, h.rootKey, sorted);
+        }
+    }
+    // the list's chunks, consecutive in the pool: taken once nothing can send the tile to another cull any
+    // more, so that a pool that holds the lists is always enough
+    const uint32_t chunks = (total + kChunk - 1) / kChunk;
+    uint32_t chunk0 = 0;
+    if (tid == 0) {
+        chunk0 = atomicAdd(&a.counters[0], chunks);
+        if (W > 1) h.first = chunk0;
+    }
+    __syncwarp();
     // the components' first positions
     uint32_t placed = 0;
     for (uint32_t b = 0; b < sorted; b += G) {
