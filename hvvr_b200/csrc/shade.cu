@@ -675,6 +675,102 @@ __device__ __forceinline__ float warpMax(float v) {
     return v;
 }
 
+// the sample's subsamples against triangle ij, then ik, given by the first nine words of their rows
+template <uint32_t N, bool FMA, int ROW>
+__device__ __forceinline__ void testRows(const ShadeSmem& sm, F3 camPos, F3 ncs, const float4& j0, const float4& j1, float j2,
+                                         uint32_t ij, const float4& k0, const float4& k1, float k2, uint32_t ik,
+                                         float (&tmax)[N], uint32_t (&hit)[N]) {
+    const V2 e0 = {pk(j0.w, k0.w), pk(j1.x, k1.x), pk(j1.y, k1.y)};
+    const V2 e1 = {pk(j1.z, k1.z), pk(j1.w, k1.w), pk(j2, k2)};
+    const V2 vr = {pk(camPos.x - j0.x, camPos.x - k0.x), pk(camPos.y - j0.y, camPos.y - k0.y),
+                   pk(camPos.z - j0.z, camPos.z - k0.z)};
+    const V2 nn = cross2(e0, e1);
+    const P2 t2 = dot2(vr, nn);
+    float tj, tk;
+    upk(t2, tj, tk);
+    const uint32_t tid = threadIdx.x;
+    const F3 du = f3(sm.dir[0][tid], sm.dir[1][tid], sm.dir[2][tid]), dv = f3(sm.dir[3][tid], sm.dir[4][tid], sm.dir[5][tid]);
+    const TriPair tp = pairSetup(nn, e0, e1, vr, V2{pk(ncs.x, ncs.x), pk(ncs.y, ncs.y), pk(ncs.z, ncs.z)},
+                                 V2{pk(du.x, du.x), pk(du.y, du.y), pk(du.z, du.z)},
+                                 V2{pk(dv.x, dv.x), pk(dv.y, dv.y), pk(dv.z, dv.z)});
+    const P2 tt = FMA ? neg2(t2) : t2;
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+        const P2 ax = *reinterpret_cast<const P2*>(&cMsaaXX[ROW][i]);
+        const P2 ay = *reinterpret_cast<const P2*>(&cMsaaYY[ROW][i]);
+        pairTest<FMA>(tp, tt, tj, tk, ij, ik, ax, ay, tmax[i], hit[i]);
+    }
+}
+
+// A list of at most kFewEntries is tested by every sample as it stands, without boxes and bounds, at up to 8
+// subsamples: their setup, and a lane's rounds over its own triangles, cost more than the tests that they save.
+// Launch alone, 1920 x 1080, one B200, with the bounds and so: a room of 14 triangles N = 1 143 and 106 us, N = 8
+// 178 and 137; 768 triangles N = 4 208 and 158; 5,600 triangles N = 8 313 and 270. Up to 64 entries the last takes
+// 248, but a textured frame over 57k triangles (N = 4) 228 us instead of 222 (218 with the bounds throughout).
+constexpr uint32_t kFewEntries = 32;
+template <uint32_t N> struct SampleHits {
+    float t[N];
+    uint32_t id[N];
+};
+// (out of line, so that the long lists' loop keeps its registers) returns how many entries pass the tile's tests
+template <uint32_t N, bool FMA, int ROW>
+__device__ __noinline__ uint32_t testFew(ShadeSmem& sm, const uint32_t* __restrict__ entries, uint32_t count,
+                                         const float4* __restrict__ tris, F3 camPos, F3 ncs, SampleHits<N>& out) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    bool keep = false;
+    if (tid < count) {
+        const uint32_t ix = __ldcg(entries + tid);
+        const float4* row = tris + 3 * size_t(ix);
+        const float4 ra = __ldg(row), rb = __ldg(row + 1), rc = __ldg(row + 2);
+        const TriGeom tri{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
+        // IntersectTriangleTile<false>::setup, FrustumPlanes::test, TestTriangleFrustaUVW != intersect_all_out
+        keep = !(dot3(camPos - tri.v0, cross3(tri.e0, tri.e1)) < 0.0f) && inFrustum(sm.pl, tri) && !uvwAllOut(sm.ro, sm.rd, tri);
+        sm.tri[tid][0] = ra;
+        sm.tri[tid][1] = rb;
+        sm.tri[tid][2] = make_float4(rc.x, __uint_as_float(ix), 0.0f, 0.0f);
+    }
+    const uint32_t kept = __ballot_sync(kFull, keep);
+    if (lane == 0) sm.need[warp][0] = kept;
+    __syncthreads();
+    float tmax[N];
+    uint32_t hit[N];
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+        tmax[i] = FLT_MAX;
+        hit[i] = ~0u;
+    }
+    // two at a time in list order; a last one alone as the pair (j, j)
+    const uint32_t groups = (count + 31u) / 32u;
+    uint32_t total = 0, g = 0, live = groups ? sm.need[0][0] : 0u, pend = ~0u;
+    for (;;) {
+        while (!live && g + 1 < groups) live = sm.need[++g][0];
+        const bool end = !live;
+        uint32_t j = pend;
+        if (!end) {
+            j = g * 32u + uint32_t(__ffs(live) - 1);
+            live &= live - 1u;
+            total++;
+            if (pend == ~0u) {
+                pend = j;
+                continue;
+            }
+        }
+        if (pend != ~0u) {
+            const float4 *a = sm.tri[pend], *b = sm.tri[j];
+            testRows<N, FMA, ROW>(sm, camPos, ncs, a[0], a[1], a[2].x, __float_as_uint(a[2].y), b[0], b[1], b[2].x,
+                                  __float_as_uint(b[2].y), tmax, hit);
+            pend = ~0u;
+        }
+        if (end) break;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+        out.t[i] = tmax[i];
+        out.id[i] = hit[i];
+    }
+    return total;
+}
+
 // One tile: intersect, G-buffer grouping, shading and resolve of its 128 samples. The tile's
 // list (TileList, chunk links, pool entries) is read through L2 (ld.cg): in a pipelined launch
 // another SM wrote it while this launch was running.
@@ -747,42 +843,44 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         du = xformDir(M, f3(b0.w, b1.x, b1.y));
         dv = xformDir(M, f3(b1.z, b1.w, b2.x));
     };
-    float dirLen;
+    const bool few = N <= 8 && L.count <= kFewEntries;
     F3 ncs; // -c
     {
         F3 c, du, dv;
         beamDirs(c, du, dv);
-        // Upper bound on |denom| / |e0 x e1| over this sample's subsamples: denom = -dir . n with
-        // dir = c + ax du + ay dv and |ax|,|ay| <= 1, so |denom| <= (|c| + |du| + |dv|) |n|.
-        dirLen = (sqrtf(dot3(c, c)) + sqrtf(dot3(du, du)) + sqrtf(dot3(dv, dv))) * 1.0001f;
-        // footprint radius: the larger singular value of (du dv)
-        const float uu = dot3(du, du), vv = dot3(dv, dv), uv = dot3(du, dv), hd = 0.5f * (uu - vv);
-        const float radius = sqrtf(0.5f * (uu + vv) + sqrtf(hd * hd + uv * uv)) * 1.00002f;
-        // (a beam that is not finite has to pass nothing by: its NaN or infinity must survive the maxima)
-        const float finite = (norm1(c) + norm1(du)) + norm1(dv);
-        const uint32_t r = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? radius : INFINITY));
-        const uint32_t d = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? dirLen : INFINITY));
-        if (tid == 0) {
-            F3 U, A, W;
-            boxAxes(du, dv, U, A, W);
-            sm.axis[0][0] = U.x; sm.axis[0][1] = U.y; sm.axis[0][2] = U.z;
-            sm.axis[1][0] = A.x; sm.axis[1][1] = A.y; sm.axis[1][2] = A.z;
-            sm.axis[2][0] = W.x; sm.axis[2][1] = W.y; sm.axis[2][2] = W.z;
-        }
-        if (lane == 0) {
-            sm.warpMax[0][warp] = __uint_as_float(r);
-            sm.warpMax[1][warp] = __uint_as_float(d);
-            sm.warpT[warp] = FLT_MAX;
-        }
         ncs = -c;
         sm.dir[0][tid] = -du.x; sm.dir[1][tid] = -du.y; sm.dir[2][tid] = -du.z;
         sm.dir[3][tid] = -dv.x; sm.dir[4][tid] = -dv.y; sm.dir[5][tid] = -dv.z;
-        __syncthreads();
-        // the warp's beams in a box along the axes
+        if (!few) {
+            // Upper bound on |denom| / |e0 x e1| over this sample's subsamples: denom = -dir . n with
+            // dir = c + ax du + ay dv and |ax|,|ay| <= 1, so |denom| <= (|c| + |du| + |dv|) |n|.
+            const float dirLen = (sqrtf(dot3(c, c)) + sqrtf(dot3(du, du)) + sqrtf(dot3(dv, dv))) * 1.0001f;
+            // footprint radius: the larger singular value of (du dv)
+            const float uu = dot3(du, du), vv = dot3(dv, dv), uv = dot3(du, dv), hd = 0.5f * (uu - vv);
+            const float radius = sqrtf(0.5f * (uu + vv) + sqrtf(hd * hd + uv * uv)) * 1.00002f;
+            // (a beam that is not finite has to pass nothing by: its NaN or infinity must survive the maxima)
+            const float finite = (norm1(c) + norm1(du)) + norm1(dv);
+            const uint32_t r = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? radius : INFINITY));
+            const uint32_t d = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? dirLen : INFINITY));
+            if (tid == 0) {
+                F3 U, A, W;
+                boxAxes(du, dv, U, A, W);
+                sm.axis[0][0] = U.x; sm.axis[0][1] = U.y; sm.axis[0][2] = U.z;
+                sm.axis[1][0] = A.x; sm.axis[1][1] = A.y; sm.axis[1][2] = A.z;
+                sm.axis[2][0] = W.x; sm.axis[2][1] = W.y; sm.axis[2][2] = W.z;
+            }
+            if (lane == 0) {
+                sm.warpMax[0][warp] = __uint_as_float(r);
+                sm.warpMax[1][warp] = __uint_as_float(d);
+                sm.warpT[warp] = FLT_MAX;
+            }
+            __syncthreads();
+            // the warp's beams in a box along the axes
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const float p = -dot3(c, f3(sm.axis[k][0], sm.axis[k][1], sm.axis[k][2])), lo = warpMin(p), hi = warpMax(p);
-            if (lane == 0) sm.box[k][warp] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * __uint_as_float(d), lo, hi);
+            for (int k = 0; k < 3; k++) {
+                const float p = -dot3(c, f3(sm.axis[k][0], sm.axis[k][1], sm.axis[k][2])), lo = warpMin(p), hi = warpMax(p);
+                if (lane == 0) sm.box[k][warp] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * __uint_as_float(d), lo, hi);
+            }
         }
     }
     float tmax[N];
@@ -793,203 +891,202 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         hit[i] = ~0u;
     }
     __syncthreads();
-    const float maxRadius = fmaxf(fmaxf(sm.warpMax[0][0], sm.warpMax[0][1]), fmaxf(sm.warpMax[0][2], sm.warpMax[0][3]));
-    const float maxLen = fmaxf(fmaxf(sm.warpMax[1][0], sm.warpMax[1][1]), fmaxf(sm.warpMax[1][2], sm.warpMax[1][3]));
-    if (tid < 3) {
-        const float lo = fminf(fminf(sm.box[tid][0].z, sm.box[tid][1].z), fminf(sm.box[tid][2].z, sm.box[tid][3].z));
-        const float hi = fmaxf(fmaxf(sm.box[tid][0].w, sm.box[tid][1].w), fmaxf(sm.box[tid][2].w, sm.box[tid][3].w));
-        sm.box[tid][4] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * maxLen, lo, hi);
-    }
-    __syncthreads();
-    SHADE_MARK(kScSetup, L.first);
-
-    // Entry tid of a chunk is copied into shared memory by cp.async (the 48-byte triangle record that its
-    // index names) while the CTA is still testing the batch before.
     const float4* __restrict__ trisG = viewPtr(V.tris);
-    uint32_t chunk = L.first, remaining = L.count; // the chunk to copy next and its entries, with all after them
-    uint32_t ready[kBatchChunks], idx[kBatchChunks]; // the copied chunks' entries, this thread's entry of each
-    auto copyBatch = [&] {
-#pragma unroll
-        for (uint32_t b = 0; b < kBatchChunks; b++) {
-            ready[b] = chunk < fr.poolChunks ? (remaining < kChunk ? remaining : kChunk) : 0u;
-            idx[b] = 0;
-            if (tid < ready[b]) {
-                idx[b] = __ldcg(fr.pool + size_t(chunk) * kChunk + tid);
-                const float4* src = trisG + 3 * size_t(idx[b]);
-                for (uint32_t k = 0; k < 3; k++) cpAsync16(&sm.tri[b * kChunk + tid][k], src + k);
-            }
-            if (ready[b]) {
-                remaining -= ready[b];
-                chunk = remaining ? __ldcg(fr.chunkNext + chunk) : kNoChunk;
-            }
-        }
-        cpAsyncCommit();
-    };
-    // Triangles that wait to be tested by this lane (kNone: none): when a lane gets a third, or the list
-    // ends, every lane tests those it has, in list order - the first in lane 0 and the second in lane 1
-    // of every packed operation (pairTest). A lone one is tested as the pair (j, j): a second test of the
-    // same triangle on the same subsample changes nothing (it either fails or writes the same depth and
-    // index again).
-    constexpr uint32_t kNone = ~0u;
-    uint32_t wait0 = kNone, wait1 = kNone;
-    float laneT = FLT_MAX; // the largest depth of the lane's subsamples
     uint32_t survivors = 0, tested = 0, lanesTested = 0;
-    copyBatch();
-    for (bool more = true; more;) {
-        // Which entries of the batch can meet the tile: the triangle's planes against the tile's box of beams
-        uint32_t kept = 0;
-        const float tileT = farther(farther(sm.warpT[0], sm.warpT[1]), farther(sm.warpT[2], sm.warpT[3]));
-        cpAsyncWaitAll();
+    if (few) {
+        SHADE_MARK(kScSetup, L.first);
+        SampleHits<N> hits;
+        lanesTested = tested = testFew<N, FMA, ROW>(sm, fr.pool + size_t(L.first) * kChunk, L.first < fr.poolChunks ? L.count : 0u, trisG,
+                                                    camPos, ncs, hits);
+        survivors = warp ? 0u : tested;
 #pragma unroll
-        for (uint32_t b = 0; b < kBatchChunks; b++) {
-            bool keep = false;
-            const uint32_t slot = b * kChunk + tid;
-            if (tid < ready[b]) {
-                const float4 ra = sm.tri[slot][0], rb = sm.tri[slot][1], rc = sm.tri[slot][2];
-                const TriGeom tri{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
-                const TriPlanes x = trianglePlanes(tri, camPos, maxRadius, maxLen);
-                if (!(x.t < 0.0f)) // IntersectTriangleTile<false>::setup
-                    keep = planesMeet(sm, 4, edgeAlong(sm, x.e[0]), edgeAlong(sm, x.e[1]), edgeAlong(sm, x.e[2]),
-                                      edgeAlong(sm, x.e[3]), x, tileT);
-            }
-            const uint32_t bal = __ballot_sync(kFull, keep);
-            if (lane == 0) sm.warpCount[b][warp] = __popc(bal);
-            kept |= (keep ? 1u : 0u) << b;
-            if (keep) sm.tri[slot][2].y = __uint_as_float(idx[b]); // (a triangle row's last three words are unused)
+        for (uint32_t i = 0; i < N; i++) {
+            tmax[i] = hits.t[i];
+            hit[i] = hits.id[i];
+        }
+        SHADE_MARK(kScTest, tested);
+#ifdef HVVR_VISIT_CLOCKS
+        ++scChunks;
+#endif
+    } else {
+        const float maxRadius = fmaxf(fmaxf(sm.warpMax[0][0], sm.warpMax[0][1]), fmaxf(sm.warpMax[0][2], sm.warpMax[0][3]));
+        const float maxLen = fmaxf(fmaxf(sm.warpMax[1][0], sm.warpMax[1][1]), fmaxf(sm.warpMax[1][2], sm.warpMax[1][3]));
+        if (tid < 3) {
+            const float lo = fminf(fminf(sm.box[tid][0].z, sm.box[tid][1].z), fminf(sm.box[tid][2].z, sm.box[tid][3].z));
+            const float hi = fmaxf(fmaxf(sm.box[tid][0].w, sm.box[tid][1].w), fmaxf(sm.box[tid][2].w, sm.box[tid][3].w));
+            sm.box[tid][4] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * maxLen, lo, hi);
         }
         __syncthreads();
-        uint32_t have = 0;
+        SHADE_MARK(kScSetup, L.first);
+
+        // Entry tid of a chunk is copied into shared memory by cp.async (the 48-byte triangle record that its
+        // index names) while the CTA is still testing the batch before.
+        uint32_t chunk = L.first, remaining = L.count; // the chunk to copy next and its entries, with all after them
+        uint32_t ready[kBatchChunks], idx[kBatchChunks]; // the copied chunks' entries, this thread's entry of each
+        auto copyBatch = [&] {
 #pragma unroll
-        for (uint32_t b = 0; b < kBatchChunks; b++) {
-            const uint32_t bal = __ballot_sync(kFull, (kept >> b) & 1u);
-            uint32_t off = have + __popc(bal & ((1u << lane) - 1u));
-#pragma unroll
-            for (uint32_t w = 0; w < 4; w++) {
-                const uint32_t cw = sm.warpCount[b][w];
-                off += (w < warp) ? cw : 0u;
-                have += cw;
-            }
-            if ((kept >> b) & 1u) sm.cand[off] = uint16_t(b * kChunk + tid);
-        }
-        __syncthreads();
-        SHADE_MARK(kScCull, have);
-        for (uint32_t first = 0; first == 0 || first < have; first += kChunk) {
-            // The tile's own tests on those, one per thread, and which warps need them. The depth bounds are
-            // the last round's; depths only fall, so they skip no triangle that could hit.
-            const uint32_t groups = first < have ? (min(have - first, kChunk) + 31u) / 32u : 0u;
-            if (warp < groups) {
-                const uint32_t js = first + tid;
-                uint32_t warps = 0;
-                if (js < have) {
-                    const uint32_t slot = sm.cand[js];
-                    const float4 ra = sm.tri[slot][0], rb = sm.tri[slot][1], rc = sm.tri[slot][2];
-                    const TriGeom tj{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
-                    const TriPlanes x = trianglePlanes(tj, camPos, maxRadius, maxLen);
-                    const F3 a0 = edgeAlong(sm, x.e[0]), a1 = edgeAlong(sm, x.e[1]), a2 = edgeAlong(sm, x.e[2]), a3 = edgeAlong(sm, x.e[3]);
-#pragma unroll
-                    for (uint32_t w = 0; w < 4; w++)
-                        if (planesMeet(sm, w, a0, a1, a2, a3, x, sm.warpT[w])) warps |= 1u << w;
-                    // FrustumPlanes::test, TestTriangleFrustaUVW != intersect_all_out
-                    if (warps && !(inFrustum(sm.pl, tj) && !uvwAllOut(sm.ro, sm.rd, tj))) warps = 0;
-                    if (warps) {
-#pragma unroll
-                        for (int e = 0; e < 4; e++) sm.edge[e][tid] = x.e[e];
-                        sm.t[tid] = x.t;
-                        sm.idx[tid] = __float_as_uint(rc.y);
-                    }
+            for (uint32_t b = 0; b < kBatchChunks; b++) {
+                ready[b] = chunk < fr.poolChunks ? (remaining < kChunk ? remaining : kChunk) : 0u;
+                idx[b] = 0;
+                if (tid < ready[b]) {
+                    idx[b] = __ldcg(fr.pool + size_t(chunk) * kChunk + tid);
+                    const float4* src = trisG + 3 * size_t(idx[b]);
+                    for (uint32_t k = 0; k < 3; k++) cpAsync16(&sm.tri[b * kChunk + tid][k], src + k);
                 }
-                survivors += __popc(__ballot_sync(kFull, warps != 0));
+                if (ready[b]) {
+                    remaining -= ready[b];
+                    chunk = remaining ? __ldcg(fr.chunkNext + chunk) : kNoChunk;
+                }
+            }
+            cpAsyncCommit();
+        };
+        // Triangles that wait to be tested by this lane (kNone: none): when a lane gets a third, or the list
+        // ends, every lane tests those it has, in list order - the first in lane 0 and the second in lane 1
+        // of every packed operation (pairTest). A lone one is tested as the pair (j, j): a second test of the
+        // same triangle on the same subsample changes nothing (it either fails or writes the same depth and
+        // index again).
+        constexpr uint32_t kNone = ~0u;
+        uint32_t wait0 = kNone, wait1 = kNone;
+        float laneT = FLT_MAX; // the largest depth of the lane's subsamples
+        copyBatch();
+        for (bool more = true; more;) {
+            // Which entries of the batch can meet the tile: the triangle's planes against the tile's box of beams
+            uint32_t kept = 0;
+            const float tileT = farther(farther(sm.warpT[0], sm.warpT[1]), farther(sm.warpT[2], sm.warpT[3]));
+            cpAsyncWaitAll();
+#pragma unroll
+            for (uint32_t b = 0; b < kBatchChunks; b++) {
+                bool keep = false;
+                const uint32_t slot = b * kChunk + tid;
+                if (tid < ready[b]) {
+                    const float4 ra = sm.tri[slot][0], rb = sm.tri[slot][1], rc = sm.tri[slot][2];
+                    const TriGeom tri{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
+                    const TriPlanes x = trianglePlanes(tri, camPos, maxRadius, maxLen);
+                    if (!(x.t < 0.0f)) // IntersectTriangleTile<false>::setup
+                        keep = planesMeet(sm, 4, edgeAlong(sm, x.e[0]), edgeAlong(sm, x.e[1]), edgeAlong(sm, x.e[2]),
+                                          edgeAlong(sm, x.e[3]), x, tileT);
+                }
+                const uint32_t bal = __ballot_sync(kFull, keep);
+                if (lane == 0) sm.warpCount[b][warp] = __popc(bal);
+                kept |= (keep ? 1u : 0u) << b;
+                if (keep) sm.tri[slot][2].y = __uint_as_float(idx[b]); // (a triangle row's last three words are unused)
+            }
+            __syncthreads();
+            uint32_t have = 0;
+#pragma unroll
+            for (uint32_t b = 0; b < kBatchChunks; b++) {
+                const uint32_t bal = __ballot_sync(kFull, (kept >> b) & 1u);
+                uint32_t off = have + __popc(bal & ((1u << lane) - 1u));
 #pragma unroll
                 for (uint32_t w = 0; w < 4; w++) {
-                    const uint32_t b = __ballot_sync(kFull, (warps >> w) & 1u);
-                    if (lane == w) sm.need[warp][w] = b;
+                    const uint32_t cw = sm.warpCount[b][w];
+                    off += (w < warp) ? cw : 0u;
+                    have += cw;
                 }
+                if ((kept >> b) & 1u) sm.cand[off] = uint16_t(b * kChunk + tid);
             }
-            const bool last = first + kChunk >= have; // (of the batch)
             __syncthreads();
-            if (last) {
-                copyBatch();
-                more = ready[0] != 0;
-            }
-            auto mayHit = [&](uint32_t slot) {
-                const float lowest = fminf(edgeValue(ncs, sm.edge[0][slot]),
-                                           fminf(edgeValue(ncs, sm.edge[1][slot]), edgeValue(ncs, sm.edge[2][slot])));
-                return !(lowest < 0.0f) && !(sm.t[slot] > laneT * edgeValue(ncs, sm.edge[3][slot]));
-            };
-            uint32_t g = 0, mine = 0; // mine: the group's triangles that the lane still has to take
-            for (;;) {
-                if (!__any_sync(kFull, mine != 0)) {
-                    if (g == groups) {
-                        if (more || !last) break;
-                    } else {
-                        // every lane decides which of its warp's triangles its own sample needs (two at a time;
-                        // an odd one twice)
-                        for (uint32_t live = sm.need[g][warp]; live;) {
-                            const uint32_t b0 = uint32_t(__ffs(live) - 1);
-                            live &= live - 1u;
-                            const uint32_t b1 = live ? uint32_t(__ffs(live) - 1) : b0;
-                            live &= live - 1u;
-                            const bool p0 = mayHit(g * 32u + b0), p1 = mayHit(g * 32u + b1);
-                            mine |= (p0 ? 1u << b0 : 0u) | (p1 ? 1u << b1 : 0u);
+            SHADE_MARK(kScCull, have);
+            for (uint32_t first = 0; first == 0 || first < have; first += kChunk) {
+                // The tile's own tests on those, one per thread, and which warps need them. The depth bounds are
+                // the last round's; depths only fall, so they skip no triangle that could hit.
+                const uint32_t groups = first < have ? (min(have - first, kChunk) + 31u) / 32u : 0u;
+                if (warp < groups) {
+                    const uint32_t js = first + tid;
+                    uint32_t warps = 0;
+                    if (js < have) {
+                        const uint32_t slot = sm.cand[js];
+                        const float4 ra = sm.tri[slot][0], rb = sm.tri[slot][1], rc = sm.tri[slot][2];
+                        const TriGeom tj{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
+                        const TriPlanes x = trianglePlanes(tj, camPos, maxRadius, maxLen);
+                        const F3 a0 = edgeAlong(sm, x.e[0]), a1 = edgeAlong(sm, x.e[1]), a2 = edgeAlong(sm, x.e[2]), a3 = edgeAlong(sm, x.e[3]);
+#pragma unroll
+                        for (uint32_t w = 0; w < 4; w++)
+                            if (planesMeet(sm, w, a0, a1, a2, a3, x, sm.warpT[w])) warps |= 1u << w;
+                        // FrustumPlanes::test, TestTriangleFrustaUVW != intersect_all_out
+                        if (warps && !(inFrustum(sm.pl, tj) && !uvwAllOut(sm.ro, sm.rd, tj))) warps = 0;
+                        if (warps) {
+#pragma unroll
+                            for (int e = 0; e < 4; e++) sm.edge[e][tid] = x.e[e];
+                            sm.t[tid] = x.t;
+                            sm.idx[tid] = __float_as_uint(rc.y);
                         }
-                        tested += __popc(__reduce_or_sync(kFull, mine));
-                        g++;
+                    }
+                    survivors += __popc(__ballot_sync(kFull, warps != 0));
+#pragma unroll
+                    for (uint32_t w = 0; w < 4; w++) {
+                        const uint32_t b = __ballot_sync(kFull, (warps >> w) & 1u);
+                        if (lane == w) sm.need[warp][w] = b;
                     }
                 }
-                // take up to two
-                for (int k = 0; k < 2; k++)
-                    if (mine && wait1 == kNone) {
-                        const uint32_t tri = sm.idx[(g - 1u) * 32u + uint32_t(__ffs(mine) - 1)];
-                        mine &= mine - 1u;
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(trisG + 3 * size_t(tri)));
-                        if (wait0 == kNone) wait0 = tri;
-                        else wait1 = tri;
-                    }
-                const bool end = g == groups && !more && last && !__any_sync(kFull, mine != 0);
-                if (__any_sync(kFull, end ? wait0 != kNone : mine != 0)) {
-                    if (wait0 != kNone) {
-                        const uint32_t ij = wait0, ik = wait1 == kNone ? wait0 : wait1;
-                        lanesTested += wait1 == kNone ? 1u : 2u;
-                        const float4* rj = trisG + 3 * size_t(ij);
-                        const float4* rk = trisG + 3 * size_t(ik);
-                        const float4 j0 = __ldg(rj), j1 = __ldg(rj + 1), k0 = __ldg(rk), k1 = __ldg(rk + 1);
-                        const float j2 = __ldg(&rj[2].x), k2 = __ldg(&rk[2].x);
-                        const V2 e0 = {pk(j0.w, k0.w), pk(j1.x, k1.x), pk(j1.y, k1.y)};
-                        const V2 e1 = {pk(j1.z, k1.z), pk(j1.w, k1.w), pk(j2, k2)};
-                        const V2 vr = {pk(camPos.x - j0.x, camPos.x - k0.x), pk(camPos.y - j0.y, camPos.y - k0.y),
-                                       pk(camPos.z - j0.z, camPos.z - k0.z)};
-                        const V2 nn = cross2(e0, e1);
-                        const P2 t2 = dot2(vr, nn);
-                        float tj, tk;
-                        upk(t2, tj, tk);
-                        const F3 du = f3(sm.dir[0][tid], sm.dir[1][tid], sm.dir[2][tid]), dv = f3(sm.dir[3][tid], sm.dir[4][tid], sm.dir[5][tid]);
-                        const TriPair tp = pairSetup(nn, e0, e1, vr, V2{pk(ncs.x, ncs.x), pk(ncs.y, ncs.y), pk(ncs.z, ncs.z)},
-                                                     V2{pk(du.x, du.x), pk(du.y, du.y), pk(du.z, du.z)},
-                                                     V2{pk(dv.x, dv.x), pk(dv.y, dv.y), pk(dv.z, dv.z)});
-                        const P2 tt = FMA ? neg2(t2) : t2;
-#pragma unroll
-                        for (uint32_t i = 0; i < N; i++) {
-                            const P2 ax = *reinterpret_cast<const P2*>(&cMsaaXX[rate][i]);
-                            const P2 ay = *reinterpret_cast<const P2*>(&cMsaaYY[rate][i]);
-                            pairTest<FMA>(tp, tt, tj, tk, ij, ik, ax, ay, tmax[i], hit[i]);
-                        }
-                        laneT = 0.0f;
-#pragma unroll
-                        for (uint32_t i = 0; i < N; i++) laneT = farther(laneT, tmax[i]);
-                        wait0 = wait1 = kNone;
-                    }
-                    __syncwarp();
+                const bool last = first + kChunk >= have; // (of the batch)
+                __syncthreads();
+                if (last) {
+                    copyBatch();
+                    more = ready[0] != 0;
                 }
-                if (end) break;
+                auto mayHit = [&](uint32_t slot) {
+                    const float lowest = fminf(edgeValue(ncs, sm.edge[0][slot]),
+                                               fminf(edgeValue(ncs, sm.edge[1][slot]), edgeValue(ncs, sm.edge[2][slot])));
+                    return !(lowest < 0.0f) && !(sm.t[slot] > laneT * edgeValue(ncs, sm.edge[3][slot]));
+                };
+                uint32_t g = 0, mine = 0; // mine: the group's triangles that the lane still has to take
+                for (;;) {
+                    if (!__any_sync(kFull, mine != 0)) {
+                        if (g == groups) {
+                            if (more || !last) break;
+                        } else {
+                            // every lane decides which of its warp's triangles its own sample needs (two at a time;
+                            // an odd one twice)
+                            for (uint32_t live = sm.need[g][warp]; live;) {
+                                const uint32_t b0 = uint32_t(__ffs(live) - 1);
+                                live &= live - 1u;
+                                const uint32_t b1 = live ? uint32_t(__ffs(live) - 1) : b0;
+                                live &= live - 1u;
+                                const bool p0 = mayHit(g * 32u + b0), p1 = mayHit(g * 32u + b1);
+                                mine |= (p0 ? 1u << b0 : 0u) | (p1 ? 1u << b1 : 0u);
+                            }
+                            tested += __popc(__reduce_or_sync(kFull, mine));
+                            g++;
+                        }
+                    }
+                    // take up to two
+                    for (int k = 0; k < 2; k++)
+                        if (mine && wait1 == kNone) {
+                            const uint32_t tri = sm.idx[(g - 1u) * 32u + uint32_t(__ffs(mine) - 1)];
+                            mine &= mine - 1u;
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(trisG + 3 * size_t(tri)));
+                            if (wait0 == kNone) wait0 = tri;
+                            else wait1 = tri;
+                        }
+                    const bool end = g == groups && !more && last && !__any_sync(kFull, mine != 0);
+                    if (__any_sync(kFull, end ? wait0 != kNone : mine != 0)) {
+                        if (wait0 != kNone) {
+                            const uint32_t ij = wait0, ik = wait1 == kNone ? wait0 : wait1;
+                            lanesTested += wait1 == kNone ? 1u : 2u;
+                            const float4* rj = trisG + 3 * size_t(ij);
+                            const float4* rk = trisG + 3 * size_t(ik);
+                            const float4 j0 = __ldg(rj), j1 = __ldg(rj + 1), k0 = __ldg(rk), k1 = __ldg(rk + 1);
+                            const float j2 = __ldg(&rj[2].x), k2 = __ldg(&rk[2].x);
+                            testRows<N, FMA, ROW>(sm, camPos, ncs, j0, j1, j2, ij, k0, k1, k2, ik, tmax, hit);
+                            laneT = 0.0f;
+#pragma unroll
+                            for (uint32_t i = 0; i < N; i++) laneT = farther(laneT, tmax[i]);
+                            wait0 = wait1 = kNone;
+                        }
+                        __syncwarp();
+                    }
+                    if (end) break;
+                }
+                const uint32_t far = __reduce_max_sync(kFull, __float_as_uint(laneT));
+                if (lane == 0) sm.warpT[warp] = __uint_as_float(far);
+                __syncthreads();
             }
-            const uint32_t far = __reduce_max_sync(kFull, __float_as_uint(laneT));
-            if (lane == 0) sm.warpT[warp] = __uint_as_float(far);
-            __syncthreads();
-        }
-        SHADE_MARK(kScTest, remaining);
+            SHADE_MARK(kScTest, remaining);
 #ifdef HVVR_VISIT_CLOCKS
-        scChunks += kBatchChunks;
+            scChunks += kBatchChunks;
 #endif
+        }
     }
 
     if (lane == 0 && survivors) atomicAdd(&fr.counters[kSurvivorWord], survivors);
