@@ -583,9 +583,14 @@ __device__ uint32_t waitReady(const uint32_t* slot, uint32_t* counters) {
 // c + ax du + ay dv: v = -dir . gv with gv = v0r x e1, w = -dir . gw with gw = e0 x v0r, and u =
 // -dir . gu with gu = n - gv - gw. Each has to have its sign bit clear, so a sample is passed by
 // when for one of the three -c . g + radius |g| + (rounding) < 0, radius bounding |ax du + ay dv| (the
-// unit offsets lie in the unit disk). The rounding term covers what the test's own operations and
+// unit offsets lie in the unit disk). With one or two subsamples the middle of their directions takes c's
+// place and half their distance (0 for one) the radius: the disk is four times the area that two need, and a
+// sample then tests little more than what it hits. The rounding term covers what the test's own operations and
 // these may be off by: S = |v0r| (|e0| + |e1|) + |n| bounds every partial result over |dir|, each of
-// the two sides loses less than 45 half-ulps of S |dir|, and flushed denormals less than the last term.
+// the two sides loses less than 45 half-ulps of S |dir| (the middle's own rounding adds 8), and flushed
+// denormals less than the last term. Launch alone with the disk and so: 57k triangles N = 1 640 x 480 137 and 85
+// us, 160 x 120 615 and 276; from far above, dozens of triangles in a pixel, N = 1 7,216 and 1,768, N = 2 7,358
+// and 6,368 (such a view was slower than without bounds: 4,106 and 4,678).
 // The test also rejects a subsample when depth * denom < t: with denom = -dir . n at most d = -c . n +
 // radius |n| + (rounding), and no subsample's depth above T, t > T d passes the sample by (with d < 0
 // no subsample sees the front; the product's rounding is inside the slack).
@@ -646,7 +651,7 @@ __device__ __forceinline__ TriPlanes trianglePlanes(const TriGeom& tri, F3 camPo
     x.t = dot3(v0r, nrm);
     const F3 gv = cross3fma(v0r, tri.e1), gw = cross3fma(tri.e0, v0r), gu = (nrm - gv) - gw;
     const float s1 = norm1(tri.e0) + norm1(tri.e1);
-    const float slack = maxLen * (6e-6f * (norm1(v0r) * s1 + norm1(nrm)) + 1e-33f * (1.0f + s1));
+    const float slack = maxLen * (7e-6f * (norm1(v0r) * s1 + norm1(nrm)) + 1e-33f * (1.0f + s1));
     x.e[0] = edgePlane(gv, radius, slack);
     x.e[1] = edgePlane(gw, radius, slack);
     x.e[2] = edgePlane(gu, radius, slack);
@@ -844,20 +849,29 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         dv = xformDir(M, f3(b1.z, b1.w, b2.x));
     };
     const bool few = N <= 8 && L.count <= kFewEntries;
-    F3 ncs; // -c
+    F3 ncs, mid; // -c, and minus the direction that the bounds are taken around
     {
         F3 c, du, dv;
         beamDirs(c, du, dv);
-        ncs = -c;
+        mid = ncs = -c;
         sm.dir[0][tid] = -du.x; sm.dir[1][tid] = -du.y; sm.dir[2][tid] = -du.z;
         sm.dir[3][tid] = -dv.x; sm.dir[4][tid] = -dv.y; sm.dir[5][tid] = -dv.z;
         if (!few) {
             // Upper bound on |denom| / |e0 x e1| over this sample's subsamples: denom = -dir . n with
             // dir = c + ax du + ay dv and |ax|,|ay| <= 1, so |denom| <= (|c| + |du| + |dv|) |n|.
             const float dirLen = (sqrtf(dot3(c, c)) + sqrtf(dot3(du, du)) + sqrtf(dot3(dv, dv))) * 1.0001f;
-            // footprint radius: the larger singular value of (du dv)
-            const float uu = dot3(du, du), vv = dot3(dv, dv), uv = dot3(du, dv), hd = 0.5f * (uu - vv);
-            const float radius = sqrtf(0.5f * (uu + vv) + sqrtf(hd * hd + uv * uv)) * 1.00002f;
+            // |ax du + ay dv| over the subsamples: the larger singular value of (du dv); of one or two, half their
+            // distance, around their middle
+            float radius;
+            if constexpr (N <= 2) {
+                const float2 o0 = cMsaa[rate][0], o1 = cMsaa[rate][N - 1];
+                mid = -(c + du * (0.5f * (o0.x + o1.x)) + dv * (0.5f * (o0.y + o1.y)));
+                const F3 half = du * (0.5f * (o0.x - o1.x)) + dv * (0.5f * (o0.y - o1.y));
+                radius = sqrtf(dot3(half, half)) * 1.00002f;
+            } else {
+                const float uu = dot3(du, du), vv = dot3(dv, dv), uv = dot3(du, dv), hd = 0.5f * (uu - vv);
+                radius = sqrtf(0.5f * (uu + vv) + sqrtf(hd * hd + uv * uv)) * 1.00002f;
+            }
             // (a beam that is not finite has to pass nothing by: its NaN or infinity must survive the maxima)
             const float finite = (norm1(c) + norm1(du)) + norm1(dv);
             const uint32_t r = __reduce_max_sync(kFull, __float_as_uint(finite <= FLT_MAX ? radius : INFINITY));
@@ -878,7 +892,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
             // the warp's beams in a box along the axes
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                const float p = -dot3(c, f3(sm.axis[k][0], sm.axis[k][1], sm.axis[k][2])), lo = warpMin(p), hi = warpMax(p);
+                const float p = dot3(mid, f3(sm.axis[k][0], sm.axis[k][1], sm.axis[k][2])), lo = warpMin(p), hi = warpMax(p);
                 if (lane == 0) sm.box[k][warp] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * __uint_as_float(d), lo, hi);
             }
         }
@@ -1026,9 +1040,9 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
                     more = ready[0] != 0;
                 }
                 auto mayHit = [&](uint32_t slot) {
-                    const float lowest = fminf(edgeValue(ncs, sm.edge[0][slot]),
-                                               fminf(edgeValue(ncs, sm.edge[1][slot]), edgeValue(ncs, sm.edge[2][slot])));
-                    return !(lowest < 0.0f) && !(sm.t[slot] > laneT * edgeValue(ncs, sm.edge[3][slot]));
+                    const float lowest = fminf(edgeValue(mid, sm.edge[0][slot]),
+                                               fminf(edgeValue(mid, sm.edge[1][slot]), edgeValue(mid, sm.edge[2][slot])));
+                    return !(lowest < 0.0f) && !(sm.t[slot] > laneT * edgeValue(mid, sm.edge[3][slot]));
                 };
                 uint32_t g = 0, mine = 0; // mine: the group's triangles that the lane still has to take
                 for (;;) {
