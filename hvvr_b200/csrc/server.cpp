@@ -592,6 +592,11 @@ int hvvr_server_add_view(hvvr_server* s, uint32_t scene, const hvvr_float_rect* 
     int r = hvvr_camera_set_samples(cam, samples, count, split);
     if (r == HVVR_OK) r = setupCamera(cam, rc->stream);
     if (r == HVVR_OK && cudaStreamSynchronize(rc->stream) != cudaSuccess) r = fail(HVVR_ERR_CUDA, "setup failed");
+    {
+        // a view is set up once: its scratch goes back, and the budget's sum of pools and instances stays whole
+        std::lock_guard<std::mutex> scratch(rc->setupScratch.mutex);
+        rc->setupScratch.buf.release();
+    }
     if (r != HVVR_OK) {
         hvvr_camera_destroy(rc, cam);
         return r;
