@@ -619,6 +619,8 @@ int cloneCamera(const hvvr_camera* src, hvvr_camera** out) {
 
 // rate groups with fewer tiles are not split
 constexpr uint32_t kSplitMinTiles = 32;
+// a frame's only rate class is not pipelined from this many tiles (enqueueFrame)
+constexpr uint32_t kUnpipedTiles = 4096;
 
 void batchConfigDefault(hvvr_batch_config* c) {
     // The sequential cull's settings, on the 1M-triangle stereo 2x1080x1200 8xMSAA frame: one-warp cull CTAs with the slowest 1/8
@@ -796,6 +798,9 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     bool first = true;
     for (auto& u : b->kevUsed) u = false;
     for (auto& u : b->kevPipelined) u = false;
+    // whether the frame has one rate class (several hide each other's launches and fill each other's gaps: a frame of
+    // 12 views in four classes took 2,050 us, and 2,120 with each class's launches as if it were alone)
+    const bool lone = std::count_if(std::begin(b->rateTiles), std::end(b->rateTiles), [](uint32_t n) { return n != 0; }) == 1;
     // the frame as the tile cull of class r sees it, `skip` tiles into the class
     auto ofClass = [](const FrameDev& f, uint32_t r, uint32_t skip) {
         FrameDev p = f;
@@ -820,9 +825,15 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             cudaStream_t ps = b->side[k];
             CUDA_TRY(cudaStreamWaitEvent(ps, b->forkEv, 0));
             if (stages) CUDA_TRY(recordStage(b->kev[k][0], ps, capturing));
-            // From 16 subsamples the shade is several times as long as the breadth-first cull, and its
-            // CTAs are better used from the cull's end, longest tile first, than waiting for tiles.
-            const bool piped = b->cfg.pipeline && (msaa < 16 || b->cfg.tile_stack_entries);
+            // Beside the breadth-first cull, whose CTAs fill the chip until it runs out of tiles, the pipeline
+            // only hides the launch between them, and costs the shades their order, longest first. It pays
+            // for a class of few tiles: 811 x 613 N = 4 (3,904 tiles) 467 us a frame piped and 489 not, 640 x 480
+            // N = 1 194 and 203, 1280 x 720 N = 2 (7,232) 1,065 and 1,073; not from 4,096 tiles, where the shade
+            // is four CTAs a slot: 960 x 540 textured N = 4 (4,096) 349 and 334, 1920 x 1080 of 14 to 5,600
+            // triangles 224 to 456 and 211 to 407, stereo 2 x 1080 x 1200 2,450 and 2,389; nor from 16
+            // subsamples, where the shade is several times as long as the cull. Classes of one frame hide each other's launches, and are piped.
+            const bool many = lone && n >= kUnpipedTiles;
+            const bool piped = b->cfg.pipeline && (b->cfg.tile_stack_entries || (msaa < 16 && !many));
             if (!lens && piped) {
                 CUDA_TRY(launchCullShadePipeline(ofClass(fr, r, p0 - rs), msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                                  fr.counters + kPipeBase + k, b->cfg.tile_cull_warps,

@@ -428,11 +428,11 @@ typedef struct {
     uint32_t timing;              /* 1: record per-stage and per-launch events (the stage, kernel and
                                      part read-backs); they cost device time (about 0.4 ms of a 6 ms
                                      stereo frame). 0 (default): the frame's start and end only */
-    uint32_t pipeline;            /* 1 (default): each part of a pinhole rate class runs its tile cull
-                                     and its intersect/shade as one pipeline - a tile is shaded as soon
-                                     as its list is complete, while other tiles are still being culled
-                                     (from 16 subsamples only with tile_stack_entries: the cull is then
-                                     a small part of the class).
+    uint32_t pipeline;            /* 1 (default): a part of a pinhole rate class may run its tile cull and its
+                                     intersect/shade as one pipeline - a tile is shaded as soon as its list is
+                                     complete. With tile_stack_entries every part does, and shades beside the
+                                     cull; beside the breadth-first cull, which fills the chip itself, only
+                                     where it pays (classes of few tiles and below 16 subsamples).
                                      0: the cull of a part finishes before its intersect/shade starts */
     uint32_t tile_cull_ctas_per_sm; /* cap on the persistent tile cull's resident CTAs per SM (0 = as many
                                      as fit): leaves room on every SM for other work (the intersect of
