@@ -217,6 +217,11 @@ struct hvvr_batch {
     bool anyLens = false;             // a thin-lens view is in the layout
     bool fpStrict = false;
     bool costValid = false;           // every view's tileCost holds a previous frame's counts
+    // what this layout's frames have shown, per rate class (learnTiles): whether they have huge tiles
+    // (0: not known), and few tiles with long lists
+    uint32_t layoutFrames = 0;
+    uint8_t hugeTiles[kRateClasses] = {};
+    bool fewLong[kRateClasses] = {};
     DevBuf<ViewDev> viewsDev;
     DevBuf<uint32_t> blockView, order, retry, ready, pool, chunkNext, counters;
     uint32_t poolChunks = 0;

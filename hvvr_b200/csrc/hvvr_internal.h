@@ -203,9 +203,10 @@ struct FrameDev {
     uint32_t* ready = nullptr;         // [tiles] ready slots of the pipelined rate classes (kReadyEmpty at frame start)
     uint32_t cullCtasPerSm = 0;        // cap on the persistent tile cull's resident CTAs per SM (0: occupancy)
     uint32_t cullPersistent = 1;       // 0: each tile-cull warp culls one tile, and the grid covers all tiles
-    uint32_t* bigCountOut = nullptr;   // [kRateClasses][2] large and huge tiles at the front of each class's order (written with it)
+    uint32_t* bigCountOut = nullptr;   // [kRateClasses][3] large, huge and split tiles at the front of each class's order (written with it)
     const uint32_t* bigCount = nullptr; // the launch's class's entries of it, and the class's tiles before the launch's first
     uint32_t bigSkip = 0;
+    uint32_t noHuge = 0;               // 1: no launch of its own for huge tiles (the class had none)
 };
 
 
@@ -228,8 +229,9 @@ enum : uint32_t {
     kTestedWord = kSurvivorWord + 1,
     kSampleTestedWord = kTestedWord + 1,
     kPipeBase = kSampleTestedWord + 1,
-    kBigBase = kPipeBase + 2 * kRateClasses, // per rate class: its large and its huge tiles (tileOrderKernel)
-    kCounterWords = kBigBase + 2 * kRateClasses
+    kBigBase = kPipeBase + 2 * kRateClasses, // per rate class kBigWords: its large, huge and split tiles (tileOrderKernel)
+    kBigWords = 3,
+    kCounterWords = kBigBase + kBigWords * kRateClasses
 };
 
 // kernel launchers (defined in the .cu files); each returns cudaGetLastError()
@@ -243,10 +245,13 @@ cudaError_t launchTileOrder(const FrameDev& fr, cudaStream_t st);
 // whose traversal stack outgrows stackLimit (0 = kTileStack; at least 8) are
 // culled again by a second launch with a 4096-entry stack.
 cudaError_t launchTileCull(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
-                           uint32_t* queues, uint32_t warps, uint32_t stackLimit, cudaStream_t st);
-// pattern: 0 the spiral, 1 the rotated grid (pinhole only; thin lens always uses the spiral)
+                           uint32_t* queues, uint32_t warps, uint32_t stackLimit, bool early, cudaStream_t st);
+// pattern: 0 the spiral, 1 the rotated grid (pinhole only; thin lens always uses the spiral). parts (pinhole,
+// nullptr: none): the word with how many of the first tiles are shaded by four CTAs each (at most kSplitTiles)
+enum : uint32_t { kSplitTiles = 256 };
 cudaError_t launchIntersectShade(const FrameDev& fr, uint32_t msaa, uint32_t pattern, bool fpStrict, bool dof,
-                                 const uint32_t* order, uint32_t first, uint32_t count, cudaStream_t st);
+                                 const uint32_t* order, uint32_t first, uint32_t count, const uint32_t* parts,
+                                 bool early, cudaStream_t st);
 // The cull -> shade pipeline of one part of a pinhole rate class over the global tiles
 // order[first, first + count), on one stream: the tile cull publishes every finished tile into fr.ready[first + i]
 // (i = the order of completion; pipe[0] counts them), and the shade launch - started while the
@@ -261,7 +266,7 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
                                uint32_t* queues, uint32_t warps, uint32_t stackLimit, uint32_t* ready,
                                uint32_t* readyTail, cudaStream_t st);
 cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
-                                    uint32_t* queues, uint32_t stackLimit, cudaStream_t st);
+                                    uint32_t* queues, uint32_t stackLimit, bool early, cudaStream_t st);
 cudaError_t launchCullShadePipeline(const FrameDev& fr, uint32_t msaa, uint32_t pattern, bool fpStrict, uint32_t first,
                                     uint32_t count, uint32_t* queues, uint32_t* pipe, uint32_t warps,
                                     uint32_t stackLimit, cudaStream_t st);

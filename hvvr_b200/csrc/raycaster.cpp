@@ -621,6 +621,8 @@ int cloneCamera(const hvvr_camera* src, hvvr_camera** out) {
 constexpr uint32_t kSplitMinTiles = 32;
 // a frame's only rate class is not pipelined from this many tiles (enqueueFrame)
 constexpr uint32_t kUnpipedTiles = 4096;
+// nor up to this many, whose cull leaves SMs free
+constexpr uint32_t kTinyTiles = 128;
 
 void batchConfigDefault(hvvr_batch_config* c) {
     // The sequential cull's settings, on the 1M-triangle stereo 2x1080x1200 8xMSAA frame: one-warp cull CTAs with the slowest 1/8
@@ -766,6 +768,23 @@ cudaError_t recordStage(cudaEvent_t ev, cudaStream_t s, bool capturing) {
 
 // Enqueues one frame on st (and the side streams, forked from and joined back to st), recording
 // the stage and per-part events (as graph nodes when capturing).
+// What the layout's frames have shown of each rate class so far, from the counters that the last finished frame
+// copied to the host. Its launches follow it from the next frame on (images do not depend on them); a class that
+// has shown huge tiles, or few tiles with long lists, keeps the launches for them, so that a view between two
+// poses does not capture its graph anew again and again. The first frame of a layout knows no costs, and the
+// host is at most two frames ahead: from the fifth the counters are a frame's that knew them.
+enum : uint8_t { kHugeUnknown, kHugeNone, kHugeSeen };
+void learnTiles(hvvr_batch* b) {
+    if (b->layoutFrames++ < 4 || !b->hostCounters) return;
+    for (uint32_t r = 0; r < kRateClasses; r++) {
+        if (!b->rateTiles[r]) continue;
+        const volatile uint32_t* w = b->hostCounters + kBigBase + kBigWords * r;
+        if (w[1]) b->hugeTiles[r] = kHugeSeen;
+        else if (b->hugeTiles[r] == kHugeUnknown) b->hugeTiles[r] = kHugeNone;
+        if (w[2]) b->fewLong[r] = true;
+    }
+}
+
 int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool capturing) {
     const bool stages = b->cfg.timing != 0;
     CUDA_TRY(recordStage(b->ev[0], st, capturing));
@@ -802,10 +821,11 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     // 12 views in four classes took 2,050 us, and 2,120 with each class's launches as if it were alone)
     const bool lone = std::count_if(std::begin(b->rateTiles), std::end(b->rateTiles), [](uint32_t n) { return n != 0; }) == 1;
     // the frame as the tile cull of class r sees it, `skip` tiles into the class
-    auto ofClass = [](const FrameDev& f, uint32_t r, uint32_t skip) {
+    auto ofClass = [&](const FrameDev& f, uint32_t r, uint32_t skip) {
         FrameDev p = f;
-        p.bigCount = f.counters + kBigBase + 2 * r;
+        p.bigCount = f.counters + kBigBase + kBigWords * r;
         p.bigSkip = skip;
+        p.noHuge = lone && b->hugeTiles[r] == kHugeNone ? 1u : 0u;
         return p;
     };
     // Pinhole classes: per part, tile cull then intersect on the part's stream, or (config.pipeline)
@@ -831,9 +851,13 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             // N = 1 194 and 203, 1280 x 720 N = 2 (7,232) 1,065 and 1,073; not from 4,096 tiles, where the shade
             // is four CTAs a slot: 960 x 540 textured N = 4 (4,096) 349 and 334, 1920 x 1080 of 14 to 5,600
             // triangles 224 to 456 and 211 to 407, stereo 2 x 1080 x 1200 2,450 and 2,389; nor from 16
-            // subsamples, where the shade is several times as long as the cull. Classes of one frame hide each other's launches, and are piped.
-            const bool many = lone && n >= kUnpipedTiles;
-            const bool piped = b->cfg.pipeline && (b->cfg.tile_stack_entries || (msaa < 16 && !many));
+            // subsamples, where the shade is several times as long as the cull, nor where a few long lists
+            // are four CTAs' each. Classes of one frame hide each other's launches, and are piped.
+            const bool many = lone && n >= kUnpipedTiles, fours = lone && b->fewLong[r] && !b->cfg.tile_stack_entries;
+            // The smallest frames are a chain of launches: each is scheduled before the one before it ends. (With
+            // more tiles the retry pass's CTAs, an SM each, would hold SMs that other CTAs have work for.)
+            const bool tiny = lone && n <= kTinyTiles && !b->cfg.tile_stack_entries, early = tiny && !lens && !stages;
+            const bool piped = b->cfg.pipeline && (b->cfg.tile_stack_entries || (msaa < 16 && !many && !fours && !tiny));
             if (!lens && piped) {
                 CUDA_TRY(launchCullShadePipeline(ofClass(fr, r, p0 - rs), msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                                  fr.counters + kPipeBase + k, b->cfg.tile_cull_warps,
@@ -852,14 +876,15 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
                 continue;
             }
             CUDA_TRY(launchTileCull(ofClass(fr, r, p0 - rs), fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
-                                    b->cfg.tile_cull_warps, b->cfg.tile_stack_entries, ps));
+                                    b->cfg.tile_cull_warps, b->cfg.tile_stack_entries, early, ps));
             if (stages) CUDA_TRY(recordStage(b->kev[k][1], ps, capturing));
             if (stages && part == 1 && first) CUDA_TRY(recordStage(b->ev[2], ps, capturing));
             if (lens) {
                 CUDA_TRY(cudaEventRecord(b->cullEv[k], ps));
                 continue;
             }
-            CUDA_TRY(launchIntersectShade(fr, msaa, pattern, b->fpStrict, false, fr.order, p0, pn, ps));
+            CUDA_TRY(launchIntersectShade(fr, msaa, pattern, b->fpStrict, false, fr.order, p0, pn,
+                                          fours ? fr.counters + kBigBase + kBigWords * r + 2 : nullptr, early, ps));
             if (stages) CUDA_TRY(recordStage(b->kev[k][2], ps, capturing));
             b->kevUsed[k] = true;
             CUDA_TRY(cudaEventRecord(b->doneEv[k], ps));
@@ -878,7 +903,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             const uint32_t k = 2 * r + 1;
             cudaStream_t ps = b->side[k];
             CUDA_TRY(cudaStreamWaitEvent(ps, b->rankEv, 0));
-            CUDA_TRY(launchIntersectShade(fr, 1u << (r % 6), 0, b->fpStrict, true, fr.order, b->rateStart[r], n, ps));
+            CUDA_TRY(launchIntersectShade(fr, 1u << (r % 6), 0, b->fpStrict, true, fr.order, b->rateStart[r], n, nullptr, false, ps));
             if (stages) CUDA_TRY(recordStage(b->kev[k][2], ps, capturing));
             b->kevUsed[k] = true;
             CUDA_TRY(cudaEventRecord(b->doneEv[k], ps));
@@ -1028,12 +1053,16 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
         TRY(reserveBatch(b, b->tiles, b->blocks, b->views.size()));
         CUDA_TRY(cudaMemcpyAsync(b->blockView.p, blockView.data(), blockView.size() * 4, cudaMemcpyHostToDevice, st));
         b->layoutKey = key;
+        b->layoutFrames = 0;
+        std::fill(std::begin(b->hugeTiles), std::end(b->hugeTiles), uint8_t(kHugeUnknown));
+        std::fill(std::begin(b->fewLong), std::end(b->fewLong), false);
         // scheduling by last frame's cost needs a previous frame of every camera in the layout
         b->costValid = std::all_of(cams.begin(), cams.end(), [](const hvvr_camera* c) { return c->costFrames > 0; });
         dropGraph(b);
     }
     TRY(ensureSideStreams(b));
     b->fpStrict = strict;
+    learnTiles(b);
 
     // this frame's view table (transforms, scene pointers), staged in pinned memory that the
     // frame before last has finished reading
@@ -1134,6 +1163,7 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
                                   uint64_t(uintptr_t(st)), b->cfg.tile_stack_entries, b->cfg.timing,
                                   b->cfg.pipeline, b->cfg.tile_cull_ctas_per_sm, b->cfg.tile_cull_persistent};
         gkey.insert(gkey.end(), std::begin(extra), std::end(extra));
+        for (uint32_t r = 0; r < kRateClasses; r++) gkey.push_back(b->hugeTiles[r] | (b->fewLong[r] ? 4u : 0u));
         if (!b->graph || gkey != b->graphKey) {
             dropGraph(b);
             CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));

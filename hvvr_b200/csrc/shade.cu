@@ -505,6 +505,16 @@ __device__ __forceinline__ bool inFrustum(const float (&pl)[4][4], const TriGeom
     return in;
 }
 
+// A long list is one CTA's: its four warps share the tile's tests and wait for one another after every batch, and
+// where triangles are far smaller than samples a batch belongs to one warp. While few tiles have long lists (the
+// order kernel's rule: at most kSplitTiles of at least 191 visits and 592 of 47, so that the chip has room) four
+// CTAs take such a tile, each for one warp's samples: a list of at least kSplitEntries is culled against that
+// warp's box alone, and nothing waits for another warp. Launch alone, one CTA and four, 57k triangles: from far above
+// N = 8 160 x 120 11,855 and 9,174 us, 640 x 480 7,705 and 4,508; N = 2 1920 x 1080 893 and 574; from near 160 x 120
+// N = 1 276 and 239. Of the longest 256 of many long lists it is slower (stereo 1,304 and 1,454, 1280 x 720 N = 32
+// 872 and 1,060), hence the rule.
+constexpr uint32_t kSplitEntries = 1024, kWhole = 4;
+
 // The list is culled kBatchChunks chunks at a time; the next ones are copied in while their samples are tested.
 constexpr uint32_t kBatchChunks = 2, kBatchSlots = kBatchChunks * kChunk;
 
@@ -545,6 +555,7 @@ template <uint32_t N> struct MinCtas { static constexpr int v = N <= 8 ? 7 : (N 
 
 // Where a shade launch takes its tiles from; item i of the launch is
 //   kFromOrder: order[first + i] (order == nullptr: first + i), i < count;
+//   kFromParts: the same, item i of the first kSplitTiles by the CTAs 4i to 4i + 3;
 //   kFromReady: the tile published in ready[first + i] by the concurrent tile cull, waited for;
 //   kFromList:  list[first + i], for i < *listCount (the retry list, counted on the device).
 struct ShadeSource {
@@ -553,6 +564,7 @@ struct ShadeSource {
     const uint32_t* list;
     const uint32_t* listCount;
     uint32_t first, count;
+    const uint32_t* parts; // kFromParts: how many of the first items have use for four CTAs
 };
 
 // Waits (one thread) until the tile cull publishes a ready slot. A wait that runs past about a
@@ -781,14 +793,18 @@ __device__ __noinline__ uint32_t testFew(ShadeSmem& sm, const uint32_t* __restri
 // another SM wrote it while this launch was running.
 // ROW: the row of the offset tables (the rate's spiral row, or + 6 for the rotated grid), a
 // compile-time constant so that the offsets stay immediate constant-bank operands
-template <uint32_t N, bool FMA, int ROW>
-__device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, ShadeSmem& sm, LightEnvDev& env, Mat4& M) {
+// SPLIT: the tile may be one of four CTAs' (kWhole: it is not), of which each tests and shades one warp's samples.
+template <uint32_t N, bool FMA, int ROW, bool SPLIT = false>
+__device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, ShadeSmem& sm, LightEnvDev& env, Mat4& M,
+                                          uint32_t part = kWhole) {
     const ViewDev& V = fr.views[fr.viewCount == 1 ? 0u : __ldg(fr.blockView + gt / kTilesPerBlock)];
     const uint32_t tile = gt - V.tileStart;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t sid = tile * kTileSize + tid;
     const uint2 lw = __ldcg(reinterpret_cast<const uint2*>(V.tileLists + tile));
     const TileList L{lw.x, lw.y};
+    const bool split = SPLIT && part != kWhole && L.count >= kSplitEntries;
+    if (SPLIT && !split && part != kWhole && part != 0) return;
     if (L.count == 0) {
         // ClearEmptyKernel (resolve.cu:527-542)
         V.colors[sid] = 0xFF000000u;
@@ -966,7 +982,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         for (bool more = true; more;) {
             // Which entries of the batch can meet the tile: the triangle's planes against the tile's box of beams
             uint32_t kept = 0;
-            const float tileT = farther(farther(sm.warpT[0], sm.warpT[1]), farther(sm.warpT[2], sm.warpT[3]));
+            const float tileT = split ? sm.warpT[part] : farther(farther(sm.warpT[0], sm.warpT[1]), farther(sm.warpT[2], sm.warpT[3]));
             cpAsyncWaitAll();
 #pragma unroll
             for (uint32_t b = 0; b < kBatchChunks; b++) {
@@ -977,7 +993,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
                     const TriGeom tri{f3(ra.x, ra.y, ra.z), f3(ra.w, rb.x, rb.y), f3(rb.z, rb.w, rc.x)};
                     const TriPlanes x = trianglePlanes(tri, camPos, maxRadius, maxLen);
                     if (!(x.t < 0.0f)) // IntersectTriangleTile<false>::setup
-                        keep = planesMeet(sm, 4, edgeAlong(sm, x.e[0]), edgeAlong(sm, x.e[1]), edgeAlong(sm, x.e[2]),
+                        keep = planesMeet(sm, split ? part : 4u, edgeAlong(sm, x.e[0]), edgeAlong(sm, x.e[1]), edgeAlong(sm, x.e[2]),
                                           edgeAlong(sm, x.e[3]), x, tileT);
                 }
                 const uint32_t bal = __ballot_sync(kFull, keep);
@@ -1016,7 +1032,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
                         const F3 a0 = edgeAlong(sm, x.e[0]), a1 = edgeAlong(sm, x.e[1]), a2 = edgeAlong(sm, x.e[2]), a3 = edgeAlong(sm, x.e[3]);
 #pragma unroll
                         for (uint32_t w = 0; w < 4; w++)
-                            if (planesMeet(sm, w, a0, a1, a2, a3, x, sm.warpT[w])) warps |= 1u << w;
+                            if ((!split || w == part) && planesMeet(sm, w, a0, a1, a2, a3, x, sm.warpT[w])) warps |= 1u << w;
                         // FrustumPlanes::test, TestTriangleFrustaUVW != intersect_all_out
                         if (warps && !(inFrustum(sm.pl, tj) && !uvwAllOut(sm.ro, sm.rd, tj))) warps = 0;
                         if (warps) {
@@ -1107,6 +1123,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
     if (lane == 0 && tested) atomicAdd(&fr.counters[kTestedWord], tested);
     lanesTested = __reduce_add_sync(kFull, lanesTested);
     if (lane == 0 && lanesTested) atomicAdd(&fr.counters[kSampleTestedWord], lanesTested);
+    if (split && warp != part) return;
     F3 c, du, dv;
     beamDirs(c, du, dv);
     if (uint32_t* hitOut = viewPtr(V.hitIds)) {
@@ -1200,16 +1217,32 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
 
 // SRC selects where the launch's tiles come from (ShadeSource): kFromOrder and kFromReady run one
 // tile per CTA; kFromList walks the list with a grid-stride loop.
-enum : int { kFromOrder = 0, kFromReady = 1, kFromList = 2 };
+enum : int { kFromOrder = 0, kFromReady = 1, kFromList = 2, kFromParts = 3 };
 
 template <uint32_t N, bool FMA, int SRC, int ROW>
 __global__ void __launch_bounds__(kTileSize, MinCtas<N>::v) intersectShadeKernel(FrameDev fr, ShadeSource src) {
     __shared__ ShadeSmem sm;
     __shared__ LightEnvDev env;
     __shared__ Mat4 M;
+    // (the cull, where this launch was scheduled before its end)
+    if constexpr (SRC == kFromOrder || SRC == kFromParts) asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (SRC == kFromOrder) {
         const uint32_t gt = src.order ? src.order[src.first + blockIdx.x] : src.first + blockIdx.x;
         shadeTile<N, FMA, ROW>(fr, gt, sm, env, M);
+    } else if constexpr (SRC == kFromParts) {
+        const uint32_t four = min(src.count, uint32_t(kSplitTiles)); // the items that have four CTAs
+        uint32_t item = blockIdx.x, part = kWhole;
+        if (item < 4 * four) {
+            part = item & 3u;
+            item >>= 2;
+            if (item >= __ldcg(src.parts)) {
+                if (part) return;
+                part = kWhole;
+            }
+        } else {
+            item -= 3 * four;
+        }
+        shadeTile<N, FMA, ROW, true>(fr, src.order[src.first + item], sm, env, M, part);
     } else if constexpr (SRC == kFromReady) {
         __shared__ uint32_t readyTile;
         if (threadIdx.x == 0) readyTile = waitReady(src.ready + src.first + blockIdx.x, fr.counters);
@@ -1587,24 +1620,39 @@ __global__ void __launch_bounds__(kTileSize) intersectShadeDofKernel(FrameDev fr
     viewPtr(V.colors)[sid] = packColor(f3(aces(rx * sN), aces(ry * sN), aces(rz * sN)));
 }
 
+// a launch over tiles in their order; parts: see launchIntersectShade; early: the launch before it in the stream is
+// the retry pass of the cull, and this one may be scheduled before that ends
+template <uint32_t N, bool FMA, int ROW>
+cudaError_t launchOrdered(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count, const uint32_t* parts,
+                          bool early, cudaStream_t st) {
+    const ShadeSource src{order, nullptr, nullptr, nullptr, first, count, parts};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(count + (parts ? 3u * std::min<uint32_t>(count, kSplitTiles) : 0u));
+    cfg.blockDim = dim3(kTileSize);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return parts ? cudaLaunchKernelEx(&cfg, intersectShadeKernel<N, FMA, kFromParts, ROW>, fr, src)
+                 : cudaLaunchKernelEx(&cfg, intersectShadeKernel<N, FMA, kFromOrder, ROW>, fr, src);
+}
+
 template <uint32_t N>
 cudaError_t launchRate(const FrameDev& fr, uint32_t pattern, bool fpStrict, bool dof, const uint32_t* order,
-                       uint32_t first, uint32_t count, cudaStream_t st) {
+                       uint32_t first, uint32_t count, const uint32_t* parts, bool early, cudaStream_t st) {
     constexpr int S = RateIndex<N>::v, G = RateIndex<N>::v + 6; // spiral / rotated-grid offset rows
     if (dof) {
         if (fpStrict) intersectShadeDofKernel<N, false><<<count, kTileSize, 0, st>>>(fr, order, first);
         else intersectShadeDofKernel<N, true><<<count, kTileSize, 0, st>>>(fr, order, first);
-    } else {
-        const ShadeSource src{order, nullptr, nullptr, nullptr, first, count};
-        if (fpStrict) {
-            if (pattern) intersectShadeKernel<N, false, kFromOrder, G><<<count, kTileSize, 0, st>>>(fr, src);
-            else intersectShadeKernel<N, false, kFromOrder, S><<<count, kTileSize, 0, st>>>(fr, src);
-        } else {
-            if (pattern) intersectShadeKernel<N, true, kFromOrder, G><<<count, kTileSize, 0, st>>>(fr, src);
-            else intersectShadeKernel<N, true, kFromOrder, S><<<count, kTileSize, 0, st>>>(fr, src);
-        }
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
+    if (fpStrict)
+        return pattern ? launchOrdered<N, false, G>(fr, order, first, count, parts, early, st)
+                       : launchOrdered<N, false, S>(fr, order, first, count, parts, early, st);
+    return pattern ? launchOrdered<N, true, G>(fr, order, first, count, parts, early, st)
+                   : launchOrdered<N, true, S>(fr, order, first, count, parts, early, st);
 }
 
 // The cull -> shade pipeline of one rate class (launchCullShadePipeline).
@@ -1624,16 +1672,16 @@ cudaError_t launchPipelineRate(const FrameDev& fr, uint32_t first, uint32_t coun
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const ShadeSource ready{nullptr, fr.ready, nullptr, nullptr, first, count};
+    const ShadeSource ready{nullptr, fr.ready, nullptr, nullptr, first, count, nullptr};
     if ((e = cudaLaunchKernelEx(&cfg, intersectShadeKernel<N, FMA, kFromReady, ROW>, fr, ready)) != cudaSuccess) return e;
     // tiles whose stack outgrew the main pass: culled again, then shaded by a small grid that walks
     // the retry list (its length is only known on the device)
-    if ((e = launchTileCullRetryPass(fr, fr.order, first, count, queues, stackLimit, st)) != cudaSuccess) return e;
+    if ((e = launchTileCullRetryPass(fr, fr.order, first, count, queues, stackLimit, false, st)) != cudaSuccess) return e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint32_t grid = std::min<uint32_t>(count, uint32_t(2 * (sms > 0 ? sms : 148)));
-    const ShadeSource retried{nullptr, nullptr, fr.retry, queues + 1, first, count};
+    const ShadeSource retried{nullptr, nullptr, fr.retry, queues + 1, first, count, nullptr};
     intersectShadeKernel<N, FMA, kFromList, ROW><<<grid, kTileSize, 0, st>>>(fr, retried);
     return cudaGetLastError();
 }
@@ -1675,15 +1723,16 @@ __global__ void remapKernel(const uint32_t* __restrict__ src, const int32_t* __r
 } // namespace
 
 cudaError_t launchIntersectShade(const FrameDev& fr, uint32_t msaa, uint32_t pattern, bool fpStrict, bool dof,
-                                 const uint32_t* order, uint32_t first, uint32_t count, cudaStream_t st) {
+                                 const uint32_t* order, uint32_t first, uint32_t count, const uint32_t* parts,
+                                 bool early, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
     switch (msaa) {
-    case 1: return launchRate<1>(fr, pattern, fpStrict, dof, order, first, count, st);
-    case 2: return launchRate<2>(fr, pattern, fpStrict, dof, order, first, count, st);
-    case 4: return launchRate<4>(fr, pattern, fpStrict, dof, order, first, count, st);
-    case 8: return launchRate<8>(fr, pattern, fpStrict, dof, order, first, count, st);
-    case 16: return launchRate<16>(fr, pattern, fpStrict, dof, order, first, count, st);
-    case 32: return launchRate<32>(fr, pattern, fpStrict, dof, order, first, count, st);
+    case 1: return launchRate<1>(fr, pattern, fpStrict, dof, order, first, count, parts, early, st);
+    case 2: return launchRate<2>(fr, pattern, fpStrict, dof, order, first, count, parts, early, st);
+    case 4: return launchRate<4>(fr, pattern, fpStrict, dof, order, first, count, parts, early, st);
+    case 8: return launchRate<8>(fr, pattern, fpStrict, dof, order, first, count, parts, early, st);
+    case 16: return launchRate<16>(fr, pattern, fpStrict, dof, order, first, count, parts, early, st);
+    case 32: return launchRate<32>(fr, pattern, fpStrict, dof, order, first, count, parts, early, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -229,7 +229,7 @@ extern "C" int hvvr_tile_cull_static(const hvvr_tile_cull_args* args, uint32_t* 
     }
     if ((e = launchWriteView(v, reinterpret_cast<ViewDev*>(scratch + kOffView), st)) != cudaSuccess)
         return failStatic(HVVR_ERR_CUDA, "view setup launch failed", e);
-    if ((e = launchTileCull(fr, nullptr, 0, tiles, scratch + kOffCounters + 4, 4, args->tile_stack_entries, st)) !=
+    if ((e = launchTileCull(fr, nullptr, 0, tiles, scratch + kOffCounters + 4, 4, args->tile_stack_entries, false, st)) !=
         cudaSuccess)
         return failStatic(HVVR_ERR_CUDA, "tile cull launch failed", e);
     scanCounts<<<1, 1024, 0, st>>>(scratch, tiles);

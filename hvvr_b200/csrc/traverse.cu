@@ -658,12 +658,13 @@ struct TileCullArgs {
     uint32_t persistent;   // 0: every warp culls one tile (the grid has a warp per tile), then exits
     const uint32_t* counts; // breadth-first cull: the large, and of those the huge, tiles at the front of the rate
                            // class's order (nullptr: none)
+    uint32_t noHuge;       // 1: the huge are culled as the large are
     uint32_t skip;         // tiles of the class before `first`
     uint32_t* bigQueue;    // work-queue head of the large tiles, zero at launch
 
     __device__ uint32_t front(uint32_t n) const { return n > skip ? min(n - skip, count) : 0u; }
     __device__ uint32_t big() const { return counts ? front(__ldcg(counts)) : 0u; }
-    __device__ uint32_t huge() const { return counts ? front(__ldcg(counts + 1)) : 0u; }
+    __device__ uint32_t huge() const { return counts && !noHuge ? front(__ldcg(counts + 1)) : 0u; }
 };
 
 // traverseTiles for one tile of view V (tile = view-local index); returns the node visits.
@@ -1642,7 +1643,9 @@ template <bool LIST>
 __global__ void __launch_bounds__(kHugeWarps * 32, 1) tileTreeHugeKernel(TileCullArgs a, uint32_t tree) {
     extern __shared__ __align__(16) unsigned char treeRaw[];
     HugeSmem& sm = *reinterpret_cast<HugeSmem*>(treeRaw);
-    if (!LIST) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (the retry pass: the cull, where the launch was scheduled before its end)
+    if (LIST) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t count = LIST ? *reinterpret_cast<volatile uint32_t*>(a.retryCount) : a.huge();
     for (uint32_t w = blockIdx.x; w < count; w += gridDim.x) {
         const uint32_t gt = LIST ? a.retry[a.first + w] : a.order[a.first + w];
@@ -1732,13 +1735,15 @@ __global__ void __launch_bounds__(1024) tileOrderKernel(FrameDev fr) {
     for (uint32_t k = 0; k < kOrderPerThread; k++) hist[tid * kOrderPerThread + k] = base + mine[k];
     __syncthreads();
     // (the exclusive prefix before the scatter moves it)
-    if (fr.bigCountOut && tid < 2 * kRateClasses) {
-        const uint32_t* h = hist + (tid >> 1) * kCostBuckets;
-        uint32_t n = h[tid & 1u ? kHugeBuckets : kBigBuckets] - h[0];
-        if (!(tid & 1u)) {
+    if (fr.bigCountOut && tid < kBigWords * kRateClasses) {
+        const uint32_t* h = hist + tid / kBigWords * kCostBuckets;
+        const uint32_t word = tid % kBigWords;
+        uint32_t n = h[word == 1 ? kHugeBuckets : kBigBuckets] - h[0];
+        if (word == 0) {
             if (h[kFewBuckets95] - h[0] <= kFewTiles) n = h[kFewBuckets95] - h[0];
             if (h[kFewBuckets47] - h[0] <= kFewTiles) n = h[kFewBuckets47] - h[0];
         }
+        if (word == 2 && (n > kSplitTiles || h[kFewBuckets47] - h[0] > kFewTiles)) n = 0;
         fr.bigCountOut[tid] = n;
     }
     __syncthreads();
@@ -1849,7 +1854,7 @@ cudaError_t launchTileTree(const TileCullArgs& a, uint32_t capPerSm, cudaStream_
     cfg.dynamicSmemBytes = sizeof(TreeSmem);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
-    if (a.counts) {
+    if (a.counts && !a.noHuge) {
         tileTreeHugeKernel<false><<<std::min<uint32_t>(a.count, d.sms), kHugeWarps * 32, sizeof(HugeSmem), st>>>(a, 1u);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         // the other tiles' cull starts beside it, once its CTAs run
@@ -1861,13 +1866,23 @@ cudaError_t launchTileTree(const TileCullArgs& a, uint32_t capPerSm, cudaStream_
     return cudaLaunchKernelEx(&cfg, tileTreeKernel, a);
 }
 
-// the retry pass: it reads the retry count on the device and exits at once when the list is empty
-cudaError_t launchTileCullRetry(const TileCullArgs& a, bool tree, cudaStream_t st) {
+// the retry pass: it reads the retry count on the device and exits at once when the list is empty. early: the
+// launch before it in the stream is the cull, and this one may be scheduled before that ends
+cudaError_t launchTileCullRetry(const TileCullArgs& a, bool tree, bool early, cudaStream_t st) {
     DeviceLimits& d = limits();
     const cudaError_t e = treeReady(d);
     if (e != cudaSuccess) return e;
-    tileTreeHugeKernel<true><<<std::min<uint32_t>(a.count, d.sms), kHugeWarps * 32, sizeof(HugeSmem), st>>>(a, tree ? 1u : 0u);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(std::min<uint32_t>(a.count, d.sms));
+    cfg.blockDim = dim3(kHugeWarps * 32);
+    cfg.dynamicSmemBytes = sizeof(HugeSmem);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, tileTreeHugeKernel<true>, a, tree ? 1u : 0u);
 }
 
 } // namespace
@@ -1891,14 +1906,14 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
     if (stackLimit == 0) {
         const TileCullArgs t{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                              order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, ready, readyTail,
-                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.bigSkip, queues + 3};
+                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.noHuge, fr.bigSkip, queues + 3};
         return launchTileTree(t, fr.cullCtasPerSm, st);
     }
     if (stackLimit > kTileStack) stackLimit = kTileStack;
     if (stackLimit < 8) return cudaErrorInvalidValue;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, queues + 2, stackLimit, ready, readyTail,
-                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, nullptr};
+                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, 0u, nullptr};
     switch (warps) {
     case 1: return launchTileCullW<1>(a, count, fr.cullCtasPerSm, st);
     case 2: return launchTileCullW<2>(a, count, fr.cullCtasPerSm, st);
@@ -1909,19 +1924,19 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
 }
 
 cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
-                                    uint32_t* queues, uint32_t stackLimit, cudaStream_t st) {
+                                    uint32_t* queues, uint32_t stackLimit, bool early, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, nullptr, nullptr, 1u,
-                         nullptr, 0u, nullptr};
-    return launchTileCullRetry(a, stackLimit == 0, st);
+                         nullptr, 0u, 0u, nullptr};
+    return launchTileCullRetry(a, stackLimit == 0, early, st);
 }
 
 cudaError_t launchTileCull(const FrameDev& fr, const uint32_t* order, uint32_t first, uint32_t count,
-                           uint32_t* queues, uint32_t warps, uint32_t stackLimit, cudaStream_t st) {
+                           uint32_t* queues, uint32_t warps, uint32_t stackLimit, bool early, cudaStream_t st) {
     const cudaError_t e = launchTileCullMain(fr, order, first, count, queues, warps, stackLimit, nullptr, nullptr, st);
     if (e != cudaSuccess) return e;
-    return launchTileCullRetryPass(fr, order, first, count, queues, stackLimit, st);
+    return launchTileCullRetryPass(fr, order, first, count, queues, stackLimit, early && stackLimit == 0, st);
 }
 
 cudaError_t launchOccupiedRank(const FrameDev& fr, cudaStream_t st) {
