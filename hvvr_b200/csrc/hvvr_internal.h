@@ -204,8 +204,7 @@ struct FrameDev {
     uint32_t cullCtasPerSm = 0;        // cap on the persistent tile cull's resident CTAs per SM (0: occupancy)
     uint32_t cullPersistent = 1;       // 0: each tile-cull warp culls one tile, and the grid covers all tiles
     uint32_t* bigCountOut = nullptr;   // [kRateClasses][3] large, huge and split tiles at the front of each class's order (written with it)
-    const uint32_t* bigCount = nullptr; // the launch's class's entries of it, and the class's tiles before the launch's first
-    uint32_t bigSkip = 0;
+    const uint32_t* bigCount = nullptr; // the launch's class's entries of it (the launch holds the class's tiles from the first)
     uint32_t noHuge = 0;               // 1: no launch of its own for huge tiles (the class had none)
 };
 
@@ -217,14 +216,14 @@ int setLastError(int code, const char* msg);
 // 12 + log2(msaa) for pinhole views with the rotated-grid pattern
 enum : uint32_t { kRateClasses = 18 };
 // counters: [0] chunk allocator, [1] status, then per tile-cull launch k (2 per rate class)
-// four words at kQueueBase + 4k: work-queue head, retry count, retry-queue head, large tiles' queue head
+// three words at kQueueBase + 3k: work-queue head, retry count, large tiles' queue head
 // then one word counting the list entries that survive the intersect's per-tile tests, one counting
 // the (warp, surviving entry) pairs of which some sample's subsample tests ran, one counting the
 // (sample, surviving entry) pairs whose subsample tests ran, then per launch part k (2 per rate class)
 // the ready-slot tail of its cull -> shade pipeline
 enum : uint32_t {
     kQueueBase = 2,
-    kQueueWords = 4,
+    kQueueWords = 3,
     kSurvivorWord = kQueueBase + kQueueWords * 2 * kRateClasses,
     kTestedWord = kSurvivorWord + 1,
     kSampleTestedWord = kTestedWord + 1,

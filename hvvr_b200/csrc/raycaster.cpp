@@ -820,11 +820,10 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     // whether the frame has one rate class (several hide each other's launches and fill each other's gaps: a frame of
     // 12 views in four classes took 2,050 us, and 2,120 with each class's launches as if it were alone)
     const bool lone = std::count_if(std::begin(b->rateTiles), std::end(b->rateTiles), [](uint32_t n) { return n != 0; }) == 1;
-    // the frame as the tile cull of class r sees it, `skip` tiles into the class
-    auto ofClass = [&](const FrameDev& f, uint32_t r, uint32_t skip) {
+    // the frame as the tile cull of class r sees it
+    auto ofClass = [&](const FrameDev& f, uint32_t r) {
         FrameDev p = f;
         p.bigCount = f.counters + kBigBase + kBigWords * r;
-        p.bigSkip = skip;
         p.noHuge = lone && b->hugeTiles[r] == kHugeNone ? 1u : 0u;
         return p;
     };
@@ -859,7 +858,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             const bool tiny = lone && n <= kTinyTiles && !b->cfg.tile_stack_entries, early = tiny && !lens && !stages;
             const bool piped = b->cfg.pipeline && (b->cfg.tile_stack_entries || (msaa < 16 && !many && !fours && !tiny));
             if (!lens && piped) {
-                CUDA_TRY(launchCullShadePipeline(ofClass(fr, r, p0 - rs), msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
+                CUDA_TRY(launchCullShadePipeline(ofClass(fr, r), msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                                  fr.counters + kPipeBase + k, b->cfg.tile_cull_warps,
                                                  b->cfg.tile_stack_entries, ps));
                 // the cull and the shade overlap: one event marks the end of both (and of the retry
@@ -875,7 +874,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
                 CUDA_TRY(cudaStreamWaitEvent(st, b->doneEv[k], 0));
                 continue;
             }
-            CUDA_TRY(launchTileCull(ofClass(fr, r, p0 - rs), fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
+            CUDA_TRY(launchTileCull(ofClass(fr, r), fr.order, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                     b->cfg.tile_cull_warps, b->cfg.tile_stack_entries, early, ps));
             if (stages) CUDA_TRY(recordStage(b->kev[k][1], ps, capturing));
             if (stages && part == 1 && first) CUDA_TRY(recordStage(b->ev[2], ps, capturing));

@@ -651,7 +651,6 @@ struct TileCullArgs {
     uint32_t* queue;       // work-queue head of this launch, zero at launch
     uint32_t* retry;       // tiles whose stack outgrew kTileStack, at retry[first + i]
     uint32_t* retryCount;  // number of such tiles, zero at launch
-    uint32_t* retryQueue;  // work-queue head of the retry pass, zero at launch
     uint32_t stackLimit;   // entries the main pass may use (<= kTileStack)
     uint32_t* ready;       // pipelined: ready slots, slot first + i for the i-th finished tile (else nullptr)
     uint32_t* readyTail;   // pipelined: finished tiles so far, zero at launch
@@ -659,12 +658,10 @@ struct TileCullArgs {
     const uint32_t* counts; // breadth-first cull: the large, and of those the huge, tiles at the front of the rate
                            // class's order (nullptr: none)
     uint32_t noHuge;       // 1: the huge are culled as the large are
-    uint32_t skip;         // tiles of the class before `first`
     uint32_t* bigQueue;    // work-queue head of the large tiles, zero at launch
 
-    __device__ uint32_t front(uint32_t n) const { return n > skip ? min(n - skip, count) : 0u; }
-    __device__ uint32_t big() const { return counts ? front(__ldcg(counts)) : 0u; }
-    __device__ uint32_t huge() const { return counts && !noHuge ? front(__ldcg(counts + 1)) : 0u; }
+    __device__ uint32_t big() const { return counts ? min(__ldcg(counts), count) : 0u; }
+    __device__ uint32_t huge() const { return counts && !noHuge ? min(__ldcg(counts + 1), count) : 0u; }
 };
 
 // traverseTiles for one tile of view V (tile = view-local index); returns the node visits.
@@ -1905,15 +1902,15 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
     if (count == 0) return cudaSuccess;
     if (stackLimit == 0) {
         const TileCullArgs t{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
-                             order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, ready, readyTail,
-                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.noHuge, fr.bigSkip, queues + 3};
+                             order, first, count, queues, fr.retry, queues + 1, kTileStack, ready, readyTail,
+                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.noHuge, queues + 2};
         return launchTileTree(t, fr.cullCtasPerSm, st);
     }
     if (stackLimit > kTileStack) stackLimit = kTileStack;
     if (stackLimit < 8) return cudaErrorInvalidValue;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
-                         order, first, count, queues, fr.retry, queues + 1, queues + 2, stackLimit, ready, readyTail,
-                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, 0u, nullptr};
+                         order, first, count, queues, fr.retry, queues + 1, stackLimit, ready, readyTail,
+                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, nullptr};
     switch (warps) {
     case 1: return launchTileCullW<1>(a, count, fr.cullCtasPerSm, st);
     case 2: return launchTileCullW<2>(a, count, fr.cullCtasPerSm, st);
@@ -1927,8 +1924,8 @@ cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, u
                                     uint32_t* queues, uint32_t stackLimit, bool early, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
-                         order, first, count, queues, fr.retry, queues + 1, queues + 2, kTileStack, nullptr, nullptr, 1u,
-                         nullptr, 0u, 0u, nullptr};
+                         order, first, count, queues, fr.retry, queues + 1, kTileStack, nullptr, nullptr, 1u,
+                         nullptr, 0u, nullptr};
     return launchTileCullRetry(a, stackLimit == 0, early, st);
 }
 
