@@ -785,6 +785,26 @@ void learnTiles(hvvr_batch* b) {
     }
 }
 
+uint32_t rateClasses(const hvvr_batch* b) {
+    return uint32_t(std::count_if(std::begin(b->rateTiles), std::end(b->rateTiles), [](uint32_t n) { return n != 0; }));
+}
+
+// Whether config.pipeline makes class r's cull and shade one pipeline.
+// Beside the breadth-first cull, whose CTAs fill the chip until it runs out of tiles, the pipeline
+// only hides the launch between them, and costs the shades their order, longest first. It pays
+// for a class of few tiles: 811 x 613 N = 4 (3,904 tiles) 467 us a frame piped and 489 not, 640 x 480
+// N = 1 194 and 203, 1280 x 720 N = 2 (7,232) 1,065 and 1,073; not from 4,096 tiles, where the shade
+// is four CTAs a slot: 960 x 540 textured N = 4 (4,096) 349 and 334, 1920 x 1080 of 14 to 5,600
+// triangles 224 to 456 and 211 to 407, stereo 2 x 1080 x 1200 2,450 and 2,389; nor from 16
+// subsamples, where the shade is several times as long as the cull, nor where a few long lists
+// are four CTAs' each. Classes of one frame hide each other's launches, and are piped.
+bool pipelines(const hvvr_batch* b, uint32_t r, bool lone) {
+    const uint32_t n = b->rateTiles[r];
+    if (!n || (r >= 6 && r < 12)) return false;
+    if (b->cfg.tile_stack_entries) return true;
+    return r % 6 < 4 && !(lone && (n >= kUnpipedTiles || n <= kTinyTiles || b->fewLong[r]));
+}
+
 int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool capturing) {
     const bool stages = b->cfg.timing != 0;
     CUDA_TRY(recordStage(b->ev[0], st, capturing));
@@ -819,7 +839,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     for (auto& u : b->kevPipelined) u = false;
     // whether the frame has one rate class (several hide each other's launches and fill each other's gaps: a frame of
     // 12 views in four classes took 2,050 us, and 2,120 with each class's launches as if it were alone)
-    const bool lone = std::count_if(std::begin(b->rateTiles), std::end(b->rateTiles), [](uint32_t n) { return n != 0; }) == 1;
+    const bool lone = rateClasses(b) == 1;
     // the frame as the tile cull of class r sees it
     auto ofClass = [&](const FrameDev& f, uint32_t r) {
         FrameDev p = f;
@@ -844,20 +864,12 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
             cudaStream_t ps = b->side[k];
             CUDA_TRY(cudaStreamWaitEvent(ps, b->forkEv, 0));
             if (stages) CUDA_TRY(recordStage(b->kev[k][0], ps, capturing));
-            // Beside the breadth-first cull, whose CTAs fill the chip until it runs out of tiles, the pipeline
-            // only hides the launch between them, and costs the shades their order, longest first. It pays
-            // for a class of few tiles: 811 x 613 N = 4 (3,904 tiles) 467 us a frame piped and 489 not, 640 x 480
-            // N = 1 194 and 203, 1280 x 720 N = 2 (7,232) 1,065 and 1,073; not from 4,096 tiles, where the shade
-            // is four CTAs a slot: 960 x 540 textured N = 4 (4,096) 349 and 334, 1920 x 1080 of 14 to 5,600
-            // triangles 224 to 456 and 211 to 407, stereo 2 x 1080 x 1200 2,450 and 2,389; nor from 16
-            // subsamples, where the shade is several times as long as the cull, nor where a few long lists
-            // are four CTAs' each. Classes of one frame hide each other's launches, and are piped.
-            const bool many = lone && n >= kUnpipedTiles, fours = lone && b->fewLong[r] && !b->cfg.tile_stack_entries;
+            const bool fours = lone && b->fewLong[r] && !b->cfg.tile_stack_entries;
             // The smallest frames are a chain of launches: each is scheduled before the one before it ends. (With
             // more tiles the retry pass's CTAs, an SM each, would hold SMs that other CTAs have work for.)
-            const bool tiny = lone && n <= kTinyTiles && !b->cfg.tile_stack_entries, early = tiny && !lens && !stages;
-            const bool piped = b->cfg.pipeline && (b->cfg.tile_stack_entries || (msaa < 16 && !many && !fours && !tiny));
-            if (!lens && piped) {
+            const bool early = lone && n <= kTinyTiles && !b->cfg.tile_stack_entries && !lens && !stages;
+            const bool piped = b->cfg.pipeline && pipelines(b, r, lone);
+            if (piped) {
                 CUDA_TRY(launchCullShadePipeline(ofClass(fr, r), msaa, pattern, b->fpStrict, p0, pn, fr.counters + kQueueBase + kQueueWords * k,
                                                  fr.counters + kPipeBase + k, b->cfg.tile_cull_warps,
                                                  b->cfg.tile_stack_entries, ps));
@@ -1535,14 +1547,30 @@ int hvvr_batch_autotune(hvvr_batch* b, uint32_t frames, hvvr_batch_config* out) 
     hvvr_batch_config best = base;
     float bestMs = INFINITY;
     uint32_t maxChunks = 0;
-    // per cull CTA width: the cull -> shade pipeline, and the split path with each heavy share
-    // (heavy_divisor 0 = no split); the pipeline does not use the heavy share
-    struct Candidate { uint32_t pipeline, div; };
-    const Candidate candidates[] = {{1u, base.heavy_divisor}, {0u, 0u}, {0u, 16u}, {0u, 8u}, {0u, 4u}};
-    for (uint32_t warps : {1u, 2u, 4u, 8u}) {
-        for (const Candidate& cand : candidates) {
+    // Per cull CTA width: the cull -> shade pipeline, and the split path with each heavy share
+    // (heavy_divisor 0 = no split); the pipeline does not use the heavy share. The breadth-first cull uses
+    // neither width nor share: with and without the pipeline, where it would make a difference.
+    struct Candidate { uint32_t warps, pipeline, div; };
+    std::vector<Candidate> candidates;
+    if (base.tile_stack_entries) {
+        for (uint32_t warps : {1u, 2u, 4u, 8u})
+            for (const Candidate& c : {Candidate{warps, 1u, base.heavy_divisor}, Candidate{warps, 0u, 0u}, Candidate{warps, 0u, 16u},
+                                       Candidate{warps, 0u, 8u}, Candidate{warps, 0u, 4u}})
+                candidates.push_back(c);
+    } else {
+        candidates = {{base.tile_cull_warps, base.pipeline, base.heavy_divisor},
+                      {base.tile_cull_warps, base.pipeline ? 0u : 1u, base.heavy_divisor}};
+    }
+    {
+        for (size_t c = 0; c < candidates.size(); c++) {
+            const Candidate& cand = candidates[c];
+            if (c && !base.tile_stack_entries) {
+                bool acts = false;
+                for (uint32_t r = 0; r < kRateClasses; r++) acts = acts || pipelines(b, r, rateClasses(b) == 1);
+                if (!acts) break;
+            }
             b->cfg = base;
-            b->cfg.tile_cull_warps = warps;
+            b->cfg.tile_cull_warps = cand.warps;
             b->cfg.pipeline = cand.pipeline;
             b->cfg.heavy_divisor = cand.div;
             std::vector<float> ms;

@@ -463,7 +463,9 @@ int hvvr_batch_set_config(hvvr_batch* batch, const hvvr_batch_config* cfg);
 /* Autotuner: renders `frames` timed frames (after one warm-up) for each tile_cull_warps in
  * {1,2,4,8} x (pipeline 1 with the configured heavy_divisor, or pipeline 0 with heavy_divisor in
  * {0,16,8,4}), keeps the fastest, then sizes the pool to 1.25x the largest list total seen (at
- * least 1M entries). Writes the chosen config to *out. */
+ * least 1M entries). Without tile_stack_entries neither tile_cull_warps nor heavy_divisor is used: then
+ * pipeline 1 and 0 are timed, or the configuration as it is where no class would be pipelined. Writes the
+ * chosen config to *out. */
 int hvvr_batch_autotune(hvvr_batch* batch, uint32_t frames, hvvr_batch_config* out);
 /* device ms of the last frame: [0] total; [1] block cull, [2] first tile cull, [3] rest of
  * cull + intersect/shade, [4] remap + copies - stages are 0 unless config.timing is 1 */
@@ -521,8 +523,8 @@ typedef struct {
     uint32_t slots;               /* batches in flight (1..8, default 2) */
     uint32_t max_batch_views;     /* views per batch (default 64) */
     uint64_t slot_list_capacity;  /* triangle-list pool entries per slot (default 256M) */
-    uint32_t tile_cull_warps;     /* as hvvr_batch_config (default 4) */
-    uint32_t heavy_divisor;       /* as hvvr_batch_config (default 8) */
+    uint32_t tile_cull_warps;     /* as hvvr_batch_config (default 4): accepted and unused, a server culls breadth */
+    uint32_t heavy_divisor;       /* as hvvr_batch_config (default 8): first, which uses neither */
     uint32_t min_batch_views;     /* with a batch in flight, wait for this many requests (default 8) ... */
     float max_wait_ms;            /* ... or until the oldest has waited this long (default 2 ms);
                                      an idle GPU takes any request at once */
