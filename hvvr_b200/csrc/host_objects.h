@@ -225,6 +225,7 @@ struct hvvr_batch {
     DevBuf<ViewDev> viewsDev;
     DevBuf<uint32_t> blockView, order, retry, ready, pool, chunkNext, counters;
     uint32_t poolChunks = 0;
+    DevBuf<uint8_t> giants;           // 25 MB of stores for the largest tiles, from the first frame that has shown some
     ViewDev* hostViews[2] = {};       // pinned staging of the per-frame view table
     size_t hostViewsCap = 0;
     cudaEvent_t hostViewsEv[2] = {};

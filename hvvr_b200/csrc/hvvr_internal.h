@@ -205,6 +205,7 @@ struct FrameDev {
     uint32_t cullPersistent = 1;       // 0: each tile-cull warp culls one tile, and the grid covers all tiles
     uint32_t* bigCountOut = nullptr;   // [kRateClasses][3] large, huge and split tiles at the front of each class's order (written with it)
     const uint32_t* bigCount = nullptr; // the launch's class's entries of it (the launch holds the class's tiles from the first)
+    void* giants = nullptr;            // stores in global memory for the largest tiles (giantStoreBytes)
     uint32_t noHuge = 0;               // 1: no launch of its own for huge tiles (the class had none)
 };
 
@@ -216,21 +217,23 @@ int setLastError(int code, const char* msg);
 // 12 + log2(msaa) for pinhole views with the rotated-grid pattern
 enum : uint32_t { kRateClasses = 18 };
 // counters: [0] chunk allocator, [1] status, then per tile-cull launch k (2 per rate class)
-// three words at kQueueBase + 3k: work-queue head, retry count, large tiles' queue head
+// five words at kQueueBase + 5k: work-queue head, retry count, large tiles' queue head, global-memory
+// stores taken, giant tiles' queue head
 // then one word counting the list entries that survive the intersect's per-tile tests, one counting
 // the (warp, surviving entry) pairs of which some sample's subsample tests ran, one counting the
 // (sample, surviving entry) pairs whose subsample tests ran, then per launch part k (2 per rate class)
 // the ready-slot tail of its cull -> shade pipeline
 enum : uint32_t {
     kQueueBase = 2,
-    kQueueWords = 3,
+    kQueueWords = 5,
     kSurvivorWord = kQueueBase + kQueueWords * 2 * kRateClasses,
     kTestedWord = kSurvivorWord + 1,
     kSampleTestedWord = kTestedWord + 1,
     kPipeBase = kSampleTestedWord + 1,
     kBigBase = kPipeBase + 2 * kRateClasses, // per rate class kBigWords: its large, huge and split tiles (tileOrderKernel)
     kBigWords = 3,
-    kCounterWords = kBigBase + kBigWords * kRateClasses
+    kGiantWord = kBigBase + kBigWords * kRateClasses, // tiles that the retry pass found above a huge tile's store
+    kCounterWords = kGiantWord + 1
 };
 
 // kernel launchers (defined in the .cu files); each returns cudaGetLastError()
@@ -248,6 +251,10 @@ cudaError_t launchTileCull(const FrameDev& fr, const uint32_t* order, uint32_t f
 // pattern: 0 the spiral, 1 the rotated grid (pinhole only; thin lens always uses the spiral). parts (pinhole,
 // nullptr: none): the word with how many of the first tiles are shaded by four CTAs each (at most kSplitTiles)
 enum : uint32_t { kSplitTiles = 256 };
+// Stores in global memory that a frame of one rate class has for its largest tiles; a retry list's entry is a
+// global tile, with kRetryGiant where it is to be culled with one.
+enum : uint32_t { kGiantSlots = 32, kRetryGiant = 0x80000000u };
+size_t giantStoreBytes();
 cudaError_t launchIntersectShade(const FrameDev& fr, uint32_t msaa, uint32_t pattern, bool fpStrict, bool dof,
                                  const uint32_t* order, uint32_t first, uint32_t count, const uint32_t* parts,
                                  bool early, cudaStream_t st);

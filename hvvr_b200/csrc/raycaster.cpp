@@ -844,6 +844,7 @@ int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool captur
     auto ofClass = [&](const FrameDev& f, uint32_t r) {
         FrameDev p = f;
         p.bigCount = f.counters + kBigBase + kBigWords * r;
+        p.giants = lone ? b->giants.p : nullptr;
         p.noHuge = lone && b->hugeTiles[r] == kHugeNone ? 1u : 0u;
         return p;
     };
@@ -1074,6 +1075,9 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
     TRY(ensureSideStreams(b));
     b->fpStrict = strict;
     learnTiles(b);
+    // (not a server's slot, whose memory is budgeted)
+    if (!b->giants.p && b->counterValid && b->hostCounters[kGiantWord] && !(b->internal && b->fixedViews))
+        TRY(b->giants.alloc(giantStoreBytes()));
 
     // this frame's view table (transforms, scene pointers), staged in pinned memory that the
     // frame before last has finished reading
@@ -1174,6 +1178,7 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
                                   uint64_t(uintptr_t(st)), b->cfg.tile_stack_entries, b->cfg.timing,
                                   b->cfg.pipeline, b->cfg.tile_cull_ctas_per_sm, b->cfg.tile_cull_persistent};
         gkey.insert(gkey.end(), std::begin(extra), std::end(extra));
+        gkey.push_back(uint64_t(uintptr_t(b->giants.p)));
         for (uint32_t r = 0; r < kRateClasses; r++) gkey.push_back(b->hugeTiles[r] | (b->fewLong[r] ? 4u : 0u));
         if (!b->graph || gkey != b->graphKey) {
             dropGraph(b);

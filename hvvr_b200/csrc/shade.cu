@@ -1253,7 +1253,7 @@ __global__ void __launch_bounds__(kTileSize, MinCtas<N>::v) intersectShadeKernel
     } else {
         const uint32_t count = *src.listCount;
         for (uint32_t item = blockIdx.x; item < count; item += gridDim.x) {
-            shadeTile<N, FMA, ROW>(fr, src.list[src.first + item], sm, env, M);
+            shadeTile<N, FMA, ROW>(fr, src.list[src.first + item] & ~kRetryGiant, sm, env, M);
             __syncthreads();
         }
     }

@@ -46,7 +46,7 @@ constexpr uint32_t kMaxChunks = 61440;                 // kMaxChunks * kChunk en
 constexpr uint64_t kMaxEntries = uint64_t(kMaxChunks) * kChunk; // 7,864,320 entries (30 MiB)
 // word layout of the scratch array
 constexpr size_t kOffCounters = 0;                     // [0] chunk allocator, [1] status, [2..3] total (u64),
-                                                       // [4..6] a launch's words (kQueueWords)
+                                                       // [4..8] a launch's words (kQueueWords)
 constexpr size_t kOffView = 64;                        // the one-view table of the cull (ViewDev)
 constexpr size_t kViewWords = (sizeof(ViewDev) + 255) / 256 * 64;
 constexpr size_t kOffLists = kOffView + kViewWords;    // TileList[kMaxTiles]
@@ -212,7 +212,7 @@ extern "C" int hvvr_tile_cull_static(const hvvr_tile_cull_args* args, uint32_t* 
     fr.poolChunks = kMaxChunks;
     fr.counters = scratch + kOffCounters;
     fr.retry = scratch + kOffRetry;
-    if ((e = cudaMemsetAsync(scratch + kOffCounters, 0, 8 * sizeof(uint32_t), st)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(scratch + kOffCounters, 0, 16 * sizeof(uint32_t), st)) != cudaSuccess)
         return failStatic(HVVR_ERR_CUDA, "clearing the scratch counters failed", e);
     {
         const uint32_t n = std::max(args->node_count, fr.blocks);

@@ -659,6 +659,9 @@ struct TileCullArgs {
                            // class's order (nullptr: none)
     uint32_t noHuge;       // 1: the huge are culled as the large are
     uint32_t* bigQueue;    // work-queue head of the large tiles, zero at launch
+    void* giants;          // kGiantSlots stores in global memory (nullptr: none), and, zero at launch,
+    uint32_t* giantSlots;  // those taken by the huge tiles' launch
+    uint32_t* giantQueue;  // work-queue head of the retry pass's giant tiles
 
     __device__ uint32_t big() const { return counts ? min(__ldcg(counts), count) : 0u; }
     __device__ uint32_t huge() const { return counts && !noHuge ? min(__ldcg(counts + 1), count) : 0u; }
@@ -966,7 +969,8 @@ __global__ void __launch_bounds__(W * 32, W == 1 ? 20 : 1) tileCullKernel(TileCu
 constexpr uint32_t kTreeWarps = 8;
 constexpr uint32_t kWarpNodes = 256;                       // visited nodes of a tile culled by one warp,
 constexpr uint32_t kCtaNodes = kTreeWarps * kWarpNodes;    // of one culled by a CTA of 8 warps,
-constexpr uint32_t kHugeWarps = 16, kHugeNodes = 8192;     // and by a CTA of 16 warps that has an SM for itself
+constexpr uint32_t kHugeWarps = 16, kHugeNodes = 8192;     // by a CTA of 16 warps that has an SM for itself,
+constexpr uint32_t kGiantNodes = 32768;                    // and by such a CTA with a store in global memory
 constexpr uint32_t kMaxGens = 64;
 constexpr uint32_t kRetryStack = 4096;
 constexpr uint32_t kMaxLeafRange = 65535;                  // longer leaf ranges are left to the sequential kernels
@@ -984,12 +988,12 @@ struct TreeStore {
     uint16_t size[N];       // nodes of the component at and below the node, then the depth-first offset
     uint16_t compSize[N];   // of heads; then the component's first position
 };
-// meta: a head's parent (bits 0-12), root index (13-18), whether its component has passing leaves
-// (19); a node's passing leaf slots (20-23) and internal children (24-26); a root that stands for
-// leaf slots only (27)
-constexpr uint32_t kMetaParent = 0x1fffu, kMetaRoot = 13, kMetaLeafy = 1u << 19, kMetaSlots = 20, kMetaChildren = 24,
-                   kMetaMasked = 1u << 27;
-static_assert(kHugeNodes <= kMetaParent + 1, "parent index bits");
+// meta: a head's parent (bits 0-14), root index (15-20), whether its component has passing leaves
+// (21); a node's passing leaf slots (22-25) and internal children (26-28); a root that stands for
+// leaf slots only (29)
+constexpr uint32_t kMetaParent = 0x7fffu, kMetaRoot = 15, kMetaLeafy = 1u << 21, kMetaSlots = 22, kMetaChildren = 26,
+                   kMetaMasked = 1u << 29;
+static_assert(kGiantNodes <= kMetaParent + 1, "parent index bits");
 static_assert(sizeof(TreeStore<kWarpNodes>::sortKey) >= sizeof(SmemFrustum), "the frustum is built in the sort's memory");
 
 struct TreeHead {
@@ -1163,7 +1167,7 @@ __device__ __noinline__ void mergeRuns(S& s, const uint32_t* rootKey, uint32_t s
 }
 
 // one tile by W warps (W = 1: the calling warp alone; else the whole CTA); returns the node visits.
-// overflow: the list was not made (see above).
+// overflow: the list was not made (see above); the return value is N where only the store was too small.
 template <int W, uint32_t N>
 __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t tile, TreeHead& h, TreeStore<N>& s,
                              bool& overflow) {
@@ -1311,7 +1315,7 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
             }
         }
         if constexpr (W == 1) {
-            if (__any_sync(kFull, bad)) next = N + 1;
+            if (__any_sync(kFull, bad)) next = kPushedBad;
             __syncwarp();
         } else {
             if (bad) atomicAdd(&h.pushed[gens % 3u], kPushedBad);
@@ -1324,7 +1328,7 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
         if (next > N || (gens >= kMaxGens && next != hi)) {
             overflow = true;
             sync();
-            return min(hi, N);
+            return next > N && next < kPushedBad ? N : min(hi, N - 1);
         }
         if (next == hi) break;
         lo = hi;
@@ -1402,7 +1406,7 @@ __device__ uint32_t treeTile(const TileCullArgs& a, const ViewDev& V, uint32_t t
     if (sorted > S::kSorted) {
         overflow = true;
         sync();
-        return visits;
+        return N;
     }
     groupSort<W>(s.sortKey, sorted, wid, sync);
     // runs of equal keys in their exact order
@@ -1632,10 +1636,16 @@ __global__ void __launch_bounds__(kTreeWarps * 32, 4) tileTreeKernel(TileCullArg
 }
 
 // The tiles that a whole SM's shared memory is for. LIST = false: the class's tiles that were this
-// large in the last frame, before its other tiles (a tile that still outgrows the store, or cannot be
-// culled breadth first, goes to the retry list). LIST = true: the retry list; what the store cannot
+// large in the last frame, before its other tiles (a tile that outgrows the store, or cannot be
+// culled breadth first, goes to the retry list). LIST = true: the retry list; what no store can
 // take, and every tile when tree is 0, is culled by one warp with the sequential traversal and the
 // reference's TileFrame capacity (4096 entries, 48 KiB).
+// A tile above kHugeNodes (a giant) has its store in global memory, of which a frame of one rate class has
+// kGiantSlots once a frame has shown such tiles: where last frame's visits say so at once, else, or with no slot
+// left, in the retry pass, marked in the list (kRetryGiant) and taken by its first kGiantSlots CTAs. Node by node
+// such a tile holds its warp, and the shade behind it, for 10 to 30 ms. Frames with the sequential kernel for them and
+// so: 1M triangles N = 8 320 x 240 17.2 and 4.6 ms, 160 x 120 29.8 and 6.7; 300k triangles from far above 1920 x 1080
+// N = 2 22.5 and 4.7.
 template <bool LIST>
 __global__ void __launch_bounds__(kHugeWarps * 32, 1) tileTreeHugeKernel(TileCullArgs a, uint32_t tree) {
     extern __shared__ __align__(16) unsigned char treeRaw[];
@@ -1643,29 +1653,74 @@ __global__ void __launch_bounds__(kHugeWarps * 32, 1) tileTreeHugeKernel(TileCul
     // (the retry pass: the cull, where the launch was scheduled before its end)
     if (LIST) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    using Giant = TreeStore<kGiantNodes>;
+    Giant* const giants = static_cast<Giant*>(a.giants);
     const uint32_t count = LIST ? *reinterpret_cast<volatile uint32_t*>(a.retryCount) : a.huge();
-    for (uint32_t w = blockIdx.x; w < count; w += gridDim.x) {
-        const uint32_t gt = LIST ? a.retry[a.first + w] : a.order[a.first + w];
-        const ViewDev& V = viewOfBlock(a.views, a.blockView, a.viewCount, gt / kTilesPerBlock);
-        const uint32_t tile = gt - V.tileStart;
-        bool overflow = true;
-        uint32_t visits = 0;
-        if (tree) {
-            visits = treeTile<kHugeWarps>(a, V, tile, sm.head, sm.cta, overflow);
-            __syncthreads();
-        }
-        if (LIST && overflow && threadIdx.x < 32) {
+    auto next = [&](uint32_t* queue) { // the queue's next number, for the CTA
+        if (threadIdx.x == 0) sm.item = atomicAdd(queue, 1u);
+        __syncthreads();
+        const uint32_t n = sm.item;
+        __syncthreads();
+        return n;
+    };
+    auto viewOf = [&](uint32_t gt) -> const ViewDev& { return viewOfBlock(a.views, a.blockView, a.viewCount, gt / kTilesPerBlock); };
+    auto giantTile = [&](const ViewDev& V, uint32_t tile, uint32_t slot, bool& overflow) {
+        const uint32_t visits = treeTile<kHugeWarps>(a, V, tile, sm.head, giants[slot], overflow);
+        __syncthreads();
+        return visits;
+    };
+    // (LIST) what no store took
+    auto sequential = [&](const ViewDev& V, uint32_t tile, uint32_t visits) {
+        if (threadIdx.x < 32) {
+            bool overflow;
             visits = cullTile(a, V, tile, sm.seq, overflow);
             if (overflow && threadIdx.x == 0) atomicOr(&a.counters[1], kStatusStackOverflow);
         }
+        return visits;
+    };
+    uint32_t slot = ~0u; // (LIST = false) the CTA's store in global memory
+    for (uint32_t w = blockIdx.x; w < count; w += gridDim.x) {
+        const uint32_t entry = LIST ? a.retry[a.first + w] : a.order[a.first + w], gt = entry & ~kRetryGiant;
+        if (LIST && entry != gt) continue; // (below)
+        const ViewDev& V = viewOf(gt);
+        const uint32_t tile = gt - V.tileStart;
+        const uint32_t last = V.tileCost[tile]; // (LIST = false: last frame's visits)
+        bool overflow = true, giant = !LIST && giants && last > kHugeNodes;
+        uint32_t visits = last;
+        if (giant) {
+            if (slot == ~0u) slot = next(a.giantSlots);
+            if (slot < kGiantSlots) {
+                visits = giantTile(V, tile, slot, overflow);
+                giant = false;
+            }
+        } else if (tree) {
+            visits = treeTile<kHugeWarps>(a, V, tile, sm.head, sm.cta, overflow);
+            giant = overflow && visits == kHugeNodes;
+            __syncthreads();
+            if (LIST && giant && threadIdx.x == 0) atomicAdd(&a.counters[kGiantWord], 1u);
+            if (LIST && giant && giants && blockIdx.x < kGiantSlots) visits = giantTile(V, tile, blockIdx.x, overflow);
+        }
+        if (LIST && overflow) visits = sequential(V, tile, visits);
         if (threadIdx.x == 0) {
             V.tileCost[tile] = visits;
             if (!LIST && overflow) {
                 V.tileLists[tile] = TileList{kNoChunk, 0};
-                a.retry[a.first + atomicAdd(a.retryCount, 1u)] = gt;
+                a.retry[a.first + atomicAdd(a.retryCount, 1u)] = gt | (giant && giants ? kRetryGiant : 0u);
             }
         }
         if (!LIST) publishTile<kHugeWarps>(a, gt, overflow);
+        __syncthreads();
+    }
+    if (!LIST || !giants || blockIdx.x >= kGiantSlots) return;
+    for (uint32_t w = next(a.giantQueue); w < count; w = next(a.giantQueue)) {
+        const uint32_t entry = a.retry[a.first + w], gt = entry & ~kRetryGiant;
+        if (entry == gt) continue;
+        const ViewDev& V = viewOf(gt);
+        const uint32_t tile = gt - V.tileStart;
+        bool overflow;
+        uint32_t visits = giantTile(V, tile, blockIdx.x, overflow);
+        if (overflow) visits = sequential(V, tile, visits);
+        if (threadIdx.x == 0) V.tileCost[tile] = visits;
         __syncthreads();
     }
 }
@@ -1884,6 +1939,8 @@ cudaError_t launchTileCullRetry(const TileCullArgs& a, bool tree, bool early, cu
 
 } // namespace
 
+size_t giantStoreBytes() { return kGiantSlots * sizeof(TreeStore<kGiantNodes>); }
+
 cudaError_t launchBlockCull(const FrameDev& fr, cudaStream_t st) {
     if (fr.blocks == 0) return cudaSuccess;
     blockCullKernel<<<fr.blocks + kPrefetchCtas, kBlockWarps * 32, 0, st>>>(fr);
@@ -1903,14 +1960,15 @@ cudaError_t launchTileCullMain(const FrameDev& fr, const uint32_t* order, uint32
     if (stackLimit == 0) {
         const TileCullArgs t{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                              order, first, count, queues, fr.retry, queues + 1, kTileStack, ready, readyTail,
-                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.noHuge, queues + 2};
+                             fr.cullPersistent ? 1u : 0u, order ? fr.bigCount : nullptr, fr.noHuge, queues + 2,
+                             fr.giants, queues + 3, queues + 4};
         return launchTileTree(t, fr.cullCtasPerSm, st);
     }
     if (stackLimit > kTileStack) stackLimit = kTileStack;
     if (stackLimit < 8) return cudaErrorInvalidValue;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, stackLimit, ready, readyTail,
-                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, nullptr};
+                         fr.cullPersistent ? 1u : 0u, nullptr, 0u, nullptr, nullptr, nullptr, nullptr};
     switch (warps) {
     case 1: return launchTileCullW<1>(a, count, fr.cullCtasPerSm, st);
     case 2: return launchTileCullW<2>(a, count, fr.cullCtasPerSm, st);
@@ -1925,7 +1983,7 @@ cudaError_t launchTileCullRetryPass(const FrameDev& fr, const uint32_t* order, u
     if (count == 0) return cudaSuccess;
     const TileCullArgs a{fr.views, fr.blockView, fr.viewCount, fr.pool, fr.chunkNext, fr.poolChunks, fr.counters,
                          order, first, count, queues, fr.retry, queues + 1, kTileStack, nullptr, nullptr, 1u,
-                         nullptr, 0u, nullptr};
+                         nullptr, 0u, nullptr, fr.giants, queues + 3, queues + 4};
     return launchTileCullRetry(a, stackLimit == 0, early, st);
 }
 
