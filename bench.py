@@ -330,6 +330,10 @@ def run_reference_arm(args, rank):
     if rank != 0:
         return
     _abi, scenes, pyoracle = library_free_imports()
+    if not pyoracle.Reference.available():
+        print(json.dumps({"impl": "reference", "unavailable": "no build of the reference's sources: oracle/_ref is made "
+                                                              "from the reference tree, which is not here"}), flush=True)
+        return
     kind, sc, smp, sessions = reference_stereo(scenes, pyoracle)
     eyes = scenes.stereo_eyes(IPD)
     cores = os.cpu_count() or 1
@@ -468,7 +472,7 @@ def main():
     # the pipeline's span and the stages, from frames with per-launch events
     _, stage_ms = launch_times(rc, cams[0], lambda k: rc.render(stream=sp), flush)
     parts = rc.part_times()
-    span = parts[2 * 3 + 1]  # rate class 3 (8x MSAA), the pipelined part
+    span = parts[2 * 3 + 1]  # rate class 3 (8x MSAA), its one part
     # each kernel alone: one launch over all tiles of the frame, serial on one stream
     kernel_ms, _ = launch_times(rc, cams[0], lambda k: rc.render(stream=sp), flush, pipeline=0, heavy_divisor=0)
     total_ms = max_over_ranks(sum(frame_ms), dist, "cuda")
@@ -526,19 +530,19 @@ def main():
                      "traffic_source": "null here: DRAM bytes per launch are in the committed ncu summaries under "
                                        "profiles/ (the BVH and the shared list triangles stay in L2, so DRAM traffic is "
                                        "far below the algorithmic bytes)",
-                     "binding_bound": "neither kernel is HBM-bound: the tile cull is latency-bound (dependent node "
-                                      "visits, see critical_path) and the intersect FP32-issue-bound (see fp32)",
+                     "binding_bound": "neither kernel is HBM-bound: the tile cull is bound by issue and the barriers "
+                                      "between generations of nodes, the intersect by issue (deciding which samples "
+                                      "need which triangles, few tests are left: see fp32) and latency",
                      "peak_source": peak_kind, "kernels": kernels, "counts": counts},
         "fp32": fp32,
-        "critical_path": {"pipeline_span_ms": float(span[2] - span[0]) if span[0] >= 0 else None,
+        "critical_path": {"cull_and_shade_span_ms": float(span[2] - span[0]) if span[0] >= 0 else None,
                           "longest_tile_node_visits": counts["longest_tile_node_visits"],
-                          "note": "the frame ends when the longest tiles' dependent node visits and their shading "
-                                  "end; span measured with per-launch events (which cost device time)"},
+                          "note": "tile cull, then intersect/shade, longest tile first; span measured with "
+                                  "per-launch events (which cost device time)"},
         "stage_ms_per_frame": {k: statistics.mean(s[i] for s in stage_ms) for i, k in
                                [(1, "block_cull"), (2, "first_tile_cull"), (3, "rest_of_cull_and_intersect_shade"),
                                 (4, "remap"), (5, "total")]},
-        # per frame: block cull, tile order, tile cull, pipelined intersect/shade, retry cull, retry-list
-        # shade, remap per eye
+        # per frame: block cull, tile order, huge tiles' cull, tile cull, retry cull, intersect/shade, remap per eye
         "gpu_launches": args.steps * 8,
         "sample_setup_ms": setup_ms,
         "clocks": ck,
@@ -1167,17 +1171,17 @@ def run_profile_case():
 
 
 VISIT_PHASES = ("row wait", "child test", "leaf refine + ranges", "multi-child insert", "next node", "list tail")
-SHADE_PHASES = ("setup", "chunk: staged triangles, tile tests, compaction", "chunk: depth skip, subsample tests",
+SHADE_PHASES = ("setup", "batch: staged triangles against the tile's box", "batch: tile and warp tests, samples' bounds and tests",
                 "outputs, G-buffer, shading")
 
 
 def run_visit_clocks():
-    """The stereo frame rendered by the profiling build of the library, whose tile cull sums the SM
-    cycles of each tile's node visits per phase (clock64 reads that wait for each phase's result)
-    and whose intersect/shade sums its CTA's cycles per phase. Prints one JSON line: cycles per
-    visit by phase for all tiles, for the slowest eighth (the heavy part) and for the 16 longest
-    tiles, and the intersect/shade cycles per tile by phase for the same sets, each from the third
-    frame after an L2 flush."""
+    """The stereo frame rendered by the profiling build of the library, whose sequential tile cull
+    (tile_stack_entries = 256) sums the SM cycles of each tile's node visits per phase (clock64 reads
+    that wait for each phase's result) and whose intersect/shade sums its CTA's cycles per phase.
+    Prints one JSON line: cycles per visit by phase for all tiles, for the slowest eighth (its heavy
+    part) and for the 16 longest tiles, and the intersect/shade cycles per tile by phase for the same
+    sets, in frames with the default, breadth-first cull; each from the third frame after an L2 flush."""
     import ctypes as C
     lib_path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "hvvr_b200", "_lib", "visit_clocks",
                             "libhvvr_b200.so")
@@ -1205,13 +1209,18 @@ def run_visit_clocks():
             cam.set_camera_to_world(xf)
             cam.set_msaa(MSAA)
             cams.append(cam)
-        for _ in range(3):
-            flush.fill_(1.0)
-            rc.render()
-        rc.synchronize()
+        def frames(stack):
+            rc.set_batch_config(tile_stack_entries=stack)
+            for _ in range(3):
+                flush.fill_(1.0)
+                rc.render()
+            rc.synchronize()
+
+        frames(256)
         tiles = sum(len(c.tile_lists()[0]) for c in cams)
         raw = np.zeros((tiles, len(VISIT_PHASES) + 1), np.uint64)
         assert lib.hvvr_dbg_visit_clocks(raw.ctypes.data, tiles) == 0
+        frames(0)
         sraw = np.zeros((tiles, len(SHADE_PHASES) + 2), np.uint64)
         assert lib.hvvr_dbg_shade_clocks(sraw.ctypes.data, tiles) == 0
     cyc, visits = raw[:, :-1].astype(np.float64), raw[:, -1].astype(np.int64)
@@ -1241,7 +1250,7 @@ def run_visit_clocks():
     top[order[:16]] = True
     stop = np.zeros(tiles, bool)
     stop[np.argsort(-scyc.sum(axis=1))[:16]] = True
-    print(json.dumps({"visit_clocks": "tile cull, stereo 2x1080x1200 8xMSAA, 995,072 triangles, frame 3 after an L2 "
+    print(json.dumps({"visit_clocks": "sequential tile cull, stereo 2x1080x1200 8xMSAA, 995,072 triangles, frame 3 after an L2 "
                                       "flush, profiling build (counters add registers and spills)",
                       "all": table(visits > 0), "slowest_eighth": table(heavy), "longest_16": table(top),
                       "longest_tile_visits": int(visits.max()),

@@ -12,13 +12,10 @@
 // All rebuild the world-space frustum of Frustum::Frustum (traverse_avx.cpp:22-211) from the
 // camera-space corner rays and the camera matrix (frustumTransform, traversal.h:38-47).
 //
-// Lane layout of one sequential node visit: lane l loads word l of the 128-byte node (one coalesced
-// row); child c = l & 3 receives its six bounds by shuffle. Lanes 0-15 run the plane test
-// of plane l>>2, lanes 16-27 the axis-projection test of axis (l-16)>>2, and every lane runs
-// one or two of the 48 edge-axis tests (edge l>>2 and, for l < 16, edge 8+(l>>2)). Ballots
-// fold the per-lane results into the reference's 4-bit child masks, so the arithmetic per
-// test is exactly the reference's lane arithmetic (explicit fmaf where it uses
-// _mm256_fmadd_ps, IEEE single ops elsewhere) and the stacks evolve identically.
+// In one sequential node visit lane l loads word l of the 128-byte node (one coalesced row) and serves one
+// test of one child, whose six bounds it receives by shuffle (LaneTest). Ballots fold the per-lane results
+// into the reference's 4-bit child masks. The arithmetic per test is the reference's lane arithmetic in every
+// kernel (explicit fmaf where it uses _mm256_fmadd_ps, IEEE single ops elsewhere), so the lists are its lists.
 #include <algorithm>
 #include <mutex>
 
