@@ -622,21 +622,27 @@ __device__ __forceinline__ F3 cross3fma(F3 a, F3 b) {
     return f3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
 }
 __device__ __forceinline__ float edgeValue(F3 nc, float4 e) { return fmaf(nc.x, e.x, fmaf(nc.y, e.y, fmaf(nc.z, e.z, e.w))); }
-// Orthonormal axes about along du and dv, to a few half-ulps whatever du and dv are: the boxes' 1e-6 of the
+__device__ __forceinline__ F3 unit(F3 v) { // (its length within 4 half-ulps of 1)
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(dot3(v, v)));
+    return v * r;
+}
+// Orthonormal axes about along du and dv, to a few half-ulps whatever du and dv are: the boxes' 2e-6 of the
 // beam length is all that their error may cost. One step of dv - U (U . dv) leaves a share of U that grows as
 // du and dv near each other (a viewport scaled very unequally under rotated ellipses), hence the second. A
-// direction lost to rounding, to squares below the normal range, or because it is zero, is replaced.
+// direction lost to rounding, to squares below the normal range, or because it is zero, is replaced. (One
+// thread's chain, which the CTA waits for: no IEEE roots and divisions.)
 __device__ __forceinline__ void boxAxes(F3 du, F3 dv, F3& U, F3& A, F3& W) {
-    U = normalize3(du);
+    U = unit(du);
     if (!(fabsf(dot3(U, U) - 1.0f) < 1e-5f)) U = f3(1.0f, 0.0f, 0.0f);
-    A = normalize3(dv - U * dot3(U, dv));
+    A = unit(dv - U * dot3(U, dv));
     A = A - U * dot3(U, A);
     if (!(dot3(A, A) > 0.5f && dot3(A, A) <= 2.0f)) { // the coordinate axis farthest from U, without its share of U
         const float x = fabsf(U.x), y = fabsf(U.y), z = fabsf(U.z);
         A = x <= y && x <= z ? f3(1.0f, 0.0f, 0.0f) : (y <= z ? f3(0.0f, 1.0f, 0.0f) : f3(0.0f, 0.0f, 1.0f));
         A = A - U * dot3(U, A);
     }
-    A = normalize3(A);
+    A = unit(A);
     W = cross3(U, A);
 }
 // a plane's components along the tile's axes, and its value over a box of beams (its largest)
@@ -909,7 +915,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const float p = dot3(mid, f3(sm.axis[k][0], sm.axis[k][1], sm.axis[k][2])), lo = warpMin(p), hi = warpMax(p);
-                if (lane == 0) sm.box[k][warp] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * __uint_as_float(d), lo, hi);
+                if (lane == 0) sm.box[k][warp] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 2e-6f * __uint_as_float(d), lo, hi);
             }
         }
     }
@@ -944,7 +950,7 @@ __device__ __forceinline__ void shadeTile(const FrameDev& fr, uint32_t gt, Shade
         if (tid < 3) {
             const float lo = fminf(fminf(sm.box[tid][0].z, sm.box[tid][1].z), fminf(sm.box[tid][2].z, sm.box[tid][3].z));
             const float hi = fmaxf(fmaxf(sm.box[tid][0].w, sm.box[tid][1].w), fmaxf(sm.box[tid][2].w, sm.box[tid][3].w));
-            sm.box[tid][4] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 1e-6f * maxLen, lo, hi);
+            sm.box[tid][4] = make_float4(0.5f * (lo + hi), 0.5f * (hi - lo) * 1.0001f + 2e-6f * maxLen, lo, hi);
         }
         __syncthreads();
         SHADE_MARK(kScSetup, L.first);
