@@ -802,7 +802,11 @@ bool pipelines(const hvvr_batch* b, uint32_t r, bool lone) {
     const uint32_t n = b->rateTiles[r];
     if (!n || (r >= 6 && r < 12)) return false;
     if (b->cfg.tile_stack_entries) return true;
-    return r % 6 < 4 && !(lone && (n >= kUnpipedTiles || n <= kTinyTiles || b->fewLong[r]));
+    if (r % 6 >= 4) return false;
+    // a cull held to fewer CTAs does leave the shade room: 1280 x 720 N = 4 over 1M triangles with one CTA an SM 1,257 us
+    // a frame piped, 1,720 not
+    if (b->cfg.tile_cull_ctas_per_sm) return true;
+    return !(lone && (n >= kUnpipedTiles || n <= kTinyTiles || b->fewLong[r]));
 }
 
 int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool capturing) {
@@ -1179,7 +1183,8 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
                                   b->cfg.pipeline, b->cfg.tile_cull_ctas_per_sm, b->cfg.tile_cull_persistent};
         gkey.insert(gkey.end(), std::begin(extra), std::end(extra));
         gkey.push_back(uint64_t(uintptr_t(b->giants.p)));
-        for (uint32_t r = 0; r < kRateClasses; r++) gkey.push_back(b->hugeTiles[r] | (b->fewLong[r] ? 4u : 0u));
+        if (rateClasses(b) == 1) // (what enqueueFrame makes of learnTiles)
+            for (uint32_t r = 0; r < kRateClasses; r++) gkey.push_back((b->hugeTiles[r] == kHugeNone ? 1u : 0u) | (b->fewLong[r] ? 2u : 0u));
         if (!b->graph || gkey != b->graphKey) {
             dropGraph(b);
             CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
