@@ -218,10 +218,10 @@ struct hvvr_batch {
     bool fpStrict = false;
     bool costValid = false;           // every view's tileCost holds a previous frame's counts
     // what this layout's frames have shown, per rate class (learnTiles): whether they have huge tiles
-    // (0: not known), and few tiles with long lists
+    // (0: not known), few tiles with long lists, and mostly large ones
     uint32_t layoutFrames = 0;
     uint8_t hugeTiles[kRateClasses] = {};
-    bool fewLong[kRateClasses] = {};
+    bool fewLong[kRateClasses] = {}, deep[kRateClasses] = {};
     DevBuf<ViewDev> viewsDev;
     DevBuf<uint32_t> blockView, order, retry, ready, pool, chunkNext, counters;
     uint32_t poolChunks = 0;

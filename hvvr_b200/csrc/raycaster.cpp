@@ -620,7 +620,7 @@ int cloneCamera(const hvvr_camera* src, hvvr_camera** out) {
 // rate groups with fewer tiles are not split
 constexpr uint32_t kSplitMinTiles = 32;
 // a frame's only rate class is not pipelined from this many tiles (enqueueFrame)
-constexpr uint32_t kUnpipedTiles = 4096;
+constexpr uint32_t kUnpipedTiles = 4096, kUnpipedDeepTiles = 8192;
 // nor up to this many, whose cull leaves SMs free
 constexpr uint32_t kTinyTiles = 128;
 
@@ -782,6 +782,7 @@ void learnTiles(hvvr_batch* b) {
         if (w[1]) b->hugeTiles[r] = kHugeSeen;
         else if (b->hugeTiles[r] == kHugeUnknown) b->hugeTiles[r] = kHugeNone;
         if (w[2]) b->fewLong[r] = true;
+        if (w[0] >= b->rateTiles[r] / 4) b->deep[r] = true;
     }
 }
 
@@ -789,15 +790,16 @@ uint32_t rateClasses(const hvvr_batch* b) {
     return uint32_t(std::count_if(std::begin(b->rateTiles), std::end(b->rateTiles), [](uint32_t n) { return n != 0; }));
 }
 
-// Whether config.pipeline makes class r's cull and shade one pipeline.
-// Beside the breadth-first cull, whose CTAs fill the chip until it runs out of tiles, the pipeline
-// only hides the launch between them, and costs the shades their order, longest first. It pays
-// for a class of few tiles: 811 x 613 N = 4 (3,904 tiles) 467 us a frame piped and 489 not, 640 x 480
-// N = 1 194 and 203, 1280 x 720 N = 2 (7,232) 1,065 and 1,073; not from 4,096 tiles, where the shade
-// is four CTAs a slot: 960 x 540 textured N = 4 (4,096) 349 and 334, 1920 x 1080 of 14 to 5,600
-// triangles 224 to 456 and 211 to 407, stereo 2 x 1080 x 1200 2,450 and 2,389; nor from 16
-// subsamples, where the shade is several times as long as the cull, nor where a few long lists
-// are four CTAs' each. Classes of one frame hide each other's launches, and are piped.
+// Whether config.pipeline makes class r's cull and shade one pipeline. Beside the breadth-first cull, whose CTAs
+// fill the chip until it runs out of tiles, the pipeline only hides the launch between them, and costs the shades
+// their order, longest first. It pays for a class of few tiles: 811 x 613 N = 4 (3,904 tiles) 467 us a frame piped
+// and 489 not, 640 x 480 N = 1 194 and 203; not from 4,096 tiles, where the shade is four CTAs a slot: 960 x 540
+// textured N = 4 (4,096) 349 and 334, 1920 x 1080 of 14 to 5,600 triangles 224 to 456 and 211 to 407, stereo
+// 2 x 1080 x 1200 2,450 and 2,389; nor from 16 subsamples, where the shade is several times as long as the cull,
+// nor where a few long lists are four CTAs' each. Where a quarter of the tiles are large, the cull is longer and
+// the line lies at 8,192: over 300k and 1M triangles 1280 x 720 (7,232 tiles) unpiped frames take 0.99 to 1.035 of
+// piped ones, and from 11,264 tiles 0.975 to 1.015 (over 57k triangles 0.955 to 0.995, and 0.91 to 0.95). Classes
+// of one frame hide each other's launches, and are piped.
 bool pipelines(const hvvr_batch* b, uint32_t r, bool lone) {
     const uint32_t n = b->rateTiles[r];
     if (!n || (r >= 6 && r < 12)) return false;
@@ -806,7 +808,7 @@ bool pipelines(const hvvr_batch* b, uint32_t r, bool lone) {
     // a cull held to fewer CTAs does leave the shade room: 1280 x 720 N = 4 over 1M triangles with one CTA an SM 1,257 us
     // a frame piped, 1,720 not
     if (b->cfg.tile_cull_ctas_per_sm) return true;
-    return !(lone && (n >= kUnpipedTiles || n <= kTinyTiles || b->fewLong[r]));
+    return !(lone && (n >= (b->deep[r] ? kUnpipedDeepTiles : kUnpipedTiles) || n <= kTinyTiles || b->fewLong[r]));
 }
 
 int enqueueFrame(hvvr_batch* b, const FrameDev& fr, cudaStream_t st, bool capturing) {
@@ -1072,6 +1074,7 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
         b->layoutFrames = 0;
         std::fill(std::begin(b->hugeTiles), std::end(b->hugeTiles), uint8_t(kHugeUnknown));
         std::fill(std::begin(b->fewLong), std::end(b->fewLong), false);
+        std::fill(std::begin(b->deep), std::end(b->deep), false);
         // scheduling by last frame's cost needs a previous frame of every camera in the layout
         b->costValid = std::all_of(cams.begin(), cams.end(), [](const hvvr_camera* c) { return c->costFrames > 0; });
         dropGraph(b);
@@ -1184,7 +1187,7 @@ int renderBatch(hvvr_batch* b, cudaStream_t st, bool skipScenes) {
         gkey.insert(gkey.end(), std::begin(extra), std::end(extra));
         gkey.push_back(uint64_t(uintptr_t(b->giants.p)));
         if (rateClasses(b) == 1) // (what enqueueFrame makes of learnTiles)
-            for (uint32_t r = 0; r < kRateClasses; r++) gkey.push_back((b->hugeTiles[r] == kHugeNone ? 1u : 0u) | (b->fewLong[r] ? 2u : 0u));
+            for (uint32_t r = 0; r < kRateClasses; r++) gkey.push_back((b->hugeTiles[r] == kHugeNone ? 1u : 0u) | (b->fewLong[r] ? 2u : 0u) | (pipelines(b, r, true) ? 4u : 0u));
         if (!b->graph || gkey != b->graphKey) {
             dropGraph(b);
             CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
