@@ -798,8 +798,9 @@ uint32_t rateClasses(const hvvr_batch* b) {
 // 2 x 1080 x 1200 2,450 and 2,389; nor from 16 subsamples, where the shade is several times as long as the cull,
 // nor where a few long lists are four CTAs' each. Where a quarter of the tiles are large, the cull is longer and
 // the line lies at 8,192: over 300k and 1M triangles 1280 x 720 (7,232 tiles) unpiped frames take 0.99 to 1.035 of
-// piped ones, and from 11,264 tiles 0.975 to 1.015 (over 57k triangles 0.955 to 0.995, and 0.91 to 0.95). Classes
-// of one frame hide each other's launches, and are piped.
+// piped ones, 1600 x 900 (11,264) 0.975 to 1.015, and 16,256 and 20,352 tiles 0.958 to 0.994 (over 57k triangles
+// 0.955 to 0.995, 0.937 to 0.951 and 0.911 to 0.940). Classes of one frame hide each other's launches, and are
+// piped.
 bool pipelines(const hvvr_batch* b, uint32_t r, bool lone) {
     const uint32_t n = b->rateTiles[r];
     if (!n || (r >= 6 && r < 12)) return false;
